@@ -120,7 +120,11 @@ SE_API se_status_t se_closure_profiled(const uint32_t* d_pref, int64_t ld_pref, 
  * of modes 5, 6 and 8, and the split-K area of modes 1, 3, 4, 6, 7 and 8: with it, for R <= 28
  * row blocks (C <= 3584), each panel tile and the next pivot tile run as 4 CTAs over disjoint
  * pivot chunks whose partial tiles the last one folds with a lane-wise max (exact), which
- * shortens each round's chain at small C. */
+ * shortens each round's chain at small C. Up to C = 1536 (16-bit lanes; 1344 in 32-bit ones) it
+ * also holds the panel buffers of the resident closure (up to 16 MiB more than the plain size):
+ * one launch that keeps the whole matrix in the SMs' registers, which the automatic schedule
+ * then runs in place of the schedules below (identical results), except into a capturing
+ * stream. */
 SE_API int64_t se_closure_workspace_bytes_flow(int C, int lane_bits, int tile);
 
 /* Task t (< R^3) of the dataflow closure's fixed order for R = ceil(C / 128) pivot blocks:
@@ -129,7 +133,9 @@ SE_API int64_t se_closure_workspace_bytes_flow(int C, int lane_bits, int tile);
 SE_API se_status_t se_closure_flow_task(uint32_t t, int R, int* kind, int* k, int* i, int* j);
 
 /* Process-wide schedule of se_closure (results are identical in every one):
- *   0  automatic (default): by C, from the variant table below; 1 where it has no entry;
+ *   0  automatic (default): the resident closure where it applies (small C, see
+ *      se_closure_workspace_bytes_flow), else by C from the variant table below; 1 where it
+ *      has no entry;
  *   1  round by round: pivot, panels and remainder launches per round, panels and pivots on
  *      the default micro-tile (8 x 8 words per thread), the next round's pivot closed by the
  *      first CTA of the remainder launch (with se_closure_workspace_bytes_flow() of workspace
@@ -162,11 +168,12 @@ SE_API se_status_t se_closure_set_mode(int mode);
 SE_API se_status_t se_closure_set_variant_table(const int* max_c, const int* modes, int n);
 
 /* The schedule (1 to 8) an se_closure call would run now for C candidates with lane_bits 16
- * or 32 and work_bytes of workspace; -1 for C < 1. Host-only. */
+ * or 32 and work_bytes of workspace; -1 for C < 1. Host-only. Where the automatic schedule
+ * runs the resident closure, this is the schedule that it stands in for. */
 SE_API int se_closure_schedule(int C, int lane_bits, int64_t work_bytes);
 
 /* Number of kernels one se_closure call launches for C candidates in 16-bit lanes under the
- * current schedule (automatic lanes add at most one more). */
+ * current schedule (automatic lanes add at most one more; the resident closure is one launch). */
 SE_API int se_closure_launch_count(int C);
 
 /* Largest C that se_closure_noalloc accepts. */

@@ -129,8 +129,9 @@ def _check_matrix(t: torch.Tensor, name: str) -> tuple[int, int]:
 def closure_workspace_bytes(num_candidates: int, lanes: int = LANES_AUTO, dataflow: bool = False) -> int:
     """Workspace bytes of the closure. dataflow=True sizes it for every schedule at its fastest:
     the dataflow form (mode 2), the second AT buffer of modes 5, 6 and 8, and the split panel
-    tiles of modes 1, 3, 4, 6, 7 and 8 up to C = 3584: a few MiB more than the
-    plain workspace. With the plain one those modes run their tiles whole, the automatic
+    tiles of modes 1, 3, 4, 6, 7 and 8 up to C = 3584, and the panel buffers of the resident
+    closure, which the automatic schedule runs up to C = 1536: a few MiB more than the
+    plain workspace (16 MiB at most). With the plain one those modes run their tiles whole, the automatic
     schedule runs 1 where it would pick 5, 6 or 8, and modes 2, 5, 6 and 8 set explicitly fail."""
     L = _lib.lib()
     fn = L.se_closure_workspace_bytes_flow if dataflow else L.se_closure_workspace_bytes
@@ -144,7 +145,8 @@ _closure_mode = 0
 
 
 def set_closure_mode(mode: int) -> None:
-    """The closure's schedule (same results in every one): 0 automatic by size (default),
+    """The closure's schedule (same results in every one): 0 automatic by size (default; up to
+    C = 1536 with the full workspace one launch that keeps the matrix in registers),
     1 round by round, 2 the dataflow form, 3 round by round with the panels on the wide
     micro-tile, 4 as 3 with each pivot tile closed by its own wide launch, 5 as 3 on two
     streams so the next round's chain overlaps the current remainder, 6 each round's

@@ -1,0 +1,31 @@
+// The one-launch closure of small matrices (closure_resident.cu), as closure.cu calls it.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "../../include/se.h"
+
+namespace se {
+namespace resident {
+
+constexpr int kB = 64;  // block edge, in cells
+
+// Largest C whose matrix fits the register files of 148 SMs: 32 x 4 tiles of 64 x 512 cells in
+// 16-bit lanes, 24 x 6 tiles of 64 x 256 cells in 32-bit lanes.
+constexpr int max_candidates(int lane_bits) { return lane_bits == 16 ? 1536 : 1344; }
+
+// Workspace bytes of the resident closure, 0 where it does not apply.
+int64_t workspace_bytes(int C, int lane_bits);
+
+// Queues the whole closure on s and sets *ran, or leaves *ran false where the resident form does
+// not apply (size, workspace, device, a capturing stream). The first two words of the workspace
+// are the closure's flags, as in closure.cu. automatic: 16-bit lanes with the window chosen on
+// the device; where none holds, word kWide is set and nothing is written to out.
+se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, int lane_bits, uint32_t base,
+                bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, bool* ran);
+
+constexpr int kWide = 4;
+
+}  // namespace resident
+}  // namespace se
