@@ -386,6 +386,13 @@ SE_API se_status_t se_tally(const int32_t* d_ids, const int64_t* d_offsets, int6
                      uint32_t* d_out, int64_t ld_out, void* d_work, int64_t work_bytes,
                      void* stream);
 
+/* se_tally that also checks the ballot index as it reads it: d_offsets must start at 0, never
+ * decrease and end at num_ids, else the call returns SE_ERR_INVALID (and d_out is undefined). No
+ * kernel follows an offset that breaks this. */
+SE_API se_status_t se_tally_checked(const int32_t* d_ids, int64_t num_ids, const int64_t* d_offsets,
+                                    int64_t V, int C, uint32_t* d_out, int64_t ld_out, void* d_work,
+                                    int64_t work_bytes, void* stream);
+
 /* se_tally without the final synchronisation: fully stream-ordered. Malformed ballots are
  * reported in the first 4 bytes of d_work (0 = fine, 2 = id out of range, 1 = lost TMA
  * completion), which the caller reads after the stream reaches that point. */

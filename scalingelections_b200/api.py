@@ -265,11 +265,6 @@ def tally_device(ids: torch.Tensor, offsets: torch.Tensor, num_candidates: int, 
     V = offsets.numel() - 1
     if V < 0:
         raise ValueError("offsets must hold V + 1 entries")
-    if V > 0:
-        # The kernels trust the CSR bounds; check them here (one small device-to-host read).
-        bad = (offsets[0] != 0) | (offsets[-1] != ids.numel()) | (offsets[1:] < offsets[:-1]).any()
-        if bool(bad):
-            raise ValueError("offsets must start at 0, never decrease and end at len(ids)")
     if out is None:
         out = torch.empty((C, C), dtype=torch.uint32, device=ids.device)
     Co, ldo = _check_matrix(out, "out")
@@ -277,8 +272,11 @@ def tally_device(ids: torch.Tensor, offsets: torch.Tensor, num_candidates: int, 
     if workspace is None or workspace.numel() * workspace.element_size() < need:
         workspace = _workspace(need, ids.device)
     with torch.cuda.device(ids.device):
-        check(_lib.lib().se_tally(ids.data_ptr(), offsets.data_ptr(), V, C, out.data_ptr(), ldo,
-                                  workspace.data_ptr(), need, _stream()))
+        status = _lib.lib().se_tally_checked(ids.data_ptr(), ids.numel(), offsets.data_ptr(), V, C, out.data_ptr(),
+                                             ldo, workspace.data_ptr(), need, _stream())
+    if status == _lib.SE_ERR_INVALID and "offsets must" in _lib.last_error():
+        raise ValueError(_lib.last_error())
+    check(status)
     return out
 
 

@@ -44,6 +44,7 @@ constexpr int kVC = 32;        // voters per TMA chunk
 constexpr int kThreads = 512;  // 8 x 4 cells per thread
 constexpr uint32_t kErrRange = 2;
 constexpr uint32_t kErrTimeout = 1;
+constexpr uint32_t kErrOffsets = 8;  // replaces any other code
 constexpr uint32_t kMaxPolls = 1u << 26;
 
 int64_t padded(int C) { return round_up(C, kTile); }
@@ -60,6 +61,22 @@ struct Irregular {
 __device__ __forceinline__ void record_irregular(const Irregular& irr, int64_t v) {
     irr.list[atomicAdd(irr.n, 1u)] = uint32_t(v);
     atomicAdd(irr.chunk + v / 32, 1u);
+}
+
+// Ballot v's span of ids. With num_ids >= 0 the offsets are checked as they are read: they must
+// start at 0, never decrease and end at num_ids. A ballot whose span breaks that is reported and
+// read as empty, so no kernel follows a bad bound; the check costs the tally no pass of its own.
+struct Span {
+    int64_t beg, len;
+    bool ok;
+};
+__device__ __forceinline__ Span ballot_span(const int64_t* offsets, int64_t id_base, int64_t v, int64_t V, int C,
+                                            int64_t num_ids) {
+    if (!offsets) return {v * C, C, true};
+    const int64_t beg = offsets[v] - id_base, end = offsets[v + 1] - id_base;
+    if (num_ids >= 0 && (beg < 0 || end < beg || end > num_ids || (v == 0 && beg != 0) || (v == V - 1 && end != num_ids)))
+        return {0, 0, false};
+    return {beg, end - beg, true};
 }
 
 // ------------------------------------------------------------------------------------------
@@ -81,11 +98,13 @@ constexpr int kPosRowMaxCq = 23552;
 template <typename Id, bool ROW>
 __global__ void __launch_bounds__(kPosThreads)
     positions_kernel(const Id* __restrict__ ids, const int64_t* __restrict__ offsets, int64_t id_base, int64_t V,
-                     int C, int64_t Cq, float* __restrict__ pos, Irregular irr, uint32_t* __restrict__ err) {
+                     int C, int64_t Cq, float* __restrict__ pos, Irregular irr, int64_t num_ids,
+                 uint32_t* __restrict__ err) {
     extern __shared__ __align__(16) uint16_t row[];
     const int64_t v = blockIdx.x;
-    const int64_t beg = offsets ? offsets[v] - id_base : v * C;
-    const int64_t len = offsets ? offsets[v + 1] - offsets[v] : C;
+    const Span span = ballot_span(offsets, id_base, v, V, C, num_ids);
+    const int64_t beg = span.beg, len = span.len;
+    if (!span.ok && threadIdx.x == 0) atomicExch(err, kErrOffsets);
     __shared__ int scratch[33];
     int code;
     if constexpr (ROW) code = block_places_u16(ids + beg, len, C, int(Cq), row, pos + v * Cq, scratch);
@@ -100,13 +119,13 @@ __global__ void __launch_bounds__(kPosThreads)
 
 template <typename Id>
 void launch_positions(const Id* ids, const int64_t* offsets, int64_t id_base, int64_t V, int C, int64_t Cq,
-                      float* pos, const Irregular& irr, uint32_t* err, cudaStream_t s) {
+                      float* pos, const Irregular& irr, int64_t num_ids, uint32_t* err, cudaStream_t s) {
     if (Cq <= kPosRowMaxCq)
         positions_kernel<Id, true><<<unsigned(V), kPosThreads, size_t(Cq) * 2, s>>>(ids, offsets, id_base, V, C, Cq,
-                                                                                 pos, irr, err);
+                                                                                 pos, irr, num_ids, err);
     else
         positions_kernel<Id, false><<<unsigned(V), kPosThreads, 0, s>>>(ids, offsets, id_base, V, C, Cq, pos, irr,
-                                                                        err);
+                                                                        num_ids, err);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -154,7 +173,7 @@ inline size_t fused_smem(int64_t Cq) { return size_t(32) * size_t(Cq + 2) * 2; }
 template <typename Id, int B>
 __global__ void __launch_bounds__(1024)
     places_planes_kernel(const Id* __restrict__ ids, const int64_t* __restrict__ offsets, int64_t id_base,
-                         int64_t V, int C, int Cq, uint32_t* __restrict__ planes, Irregular irr,
+                         int64_t V, int C, int Cq, uint32_t* __restrict__ planes, Irregular irr, int64_t num_ids,
                          uint32_t* __restrict__ err) {
     extern __shared__ __align__(16) uint16_t rows[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -163,9 +182,9 @@ __global__ void __launch_bounds__(1024)
     const int64_t v = ch * 32 + warp;
     uint16_t* row = rows + warp * pitch;
     if (v < V) {
-        const int64_t beg = offsets ? offsets[v] - id_base : v * C;
-        const int64_t len = offsets ? offsets[v + 1] - offsets[v] : C;
-        const int code = warp_places_u16(ids + beg, len, C, Cq, row);
+        const Span span = ballot_span(offsets, id_base, v, V, C, num_ids);
+        if (!span.ok && lane == 0) atomicExch(err, kErrOffsets);
+        const int code = warp_places_u16(ids + span.beg, span.len, C, Cq, row);
         if (code == kPosRepeat) {  // an irregular ballot: place 0 everywhere, counted apart
             __syncwarp();
             for (int c = lane; c < Cq; c += 32) row[c] = 0;
@@ -457,7 +476,8 @@ __global__ void __launch_bounds__(kIrrThreads)
 
 // The pack and count kernels for each plane count 1 .. kMaxPlanes.
 template <typename Id>
-using FusedKernel = void (*)(const Id*, const int64_t*, int64_t, int64_t, int, int, uint32_t*, Irregular, uint32_t*);
+using FusedKernel = void (*)(const Id*, const int64_t*, int64_t, int64_t, int, int, uint32_t*, Irregular, int64_t,
+                             uint32_t*);
 
 struct TallyKernels {
     void (*pack)(const float*, int64_t, int64_t, uint32_t*);
@@ -514,7 +534,7 @@ extern "C" int64_t se_tally_workspace_bytes(int64_t V, int C) {
 namespace {
 se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets, int64_t id_base, int64_t V, int C,
                        unsigned flags, uint32_t* d_out, int64_t ld_out, void* d_work, int64_t work_bytes,
-                       void* stream_) {
+                       void* stream_, int64_t num_ids = -1) {
     clear_error();
     SE_REQUIRE(C >= 1 && C <= (1 << 20), SE_ERR_INVALID, "Number of candidates out of range (%d)", C);
     SE_REQUIRE(V >= 0 && V < (int64_t(1) << 24), SE_ERR_INVALID, "Number of voters out of range (%lld)",
@@ -566,21 +586,24 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
         if (se_status_t st = raise_smem_limit(fn, int(fused_smem(kFusedMaxCq)), "the places kernel")) return st;
         if (w == 0)
             K.fused8<<<unsigned(nch_all), 1024, smem, s>>>(static_cast<const uint8_t*>(d_ids), d_offsets, id_base, V, C,
-                                                           int(Cq), planes, irr, err);
+                                                           int(Cq), planes, irr, num_ids, err);
         else if (w == 1)
             K.fused16<<<unsigned(nch_all), 1024, smem, s>>>(static_cast<const uint16_t*>(d_ids), d_offsets, id_base, V,
-                                                            C, int(Cq), planes, irr, err);
+                                                            C, int(Cq), planes, irr, num_ids, err);
         else
             K.fused32<<<unsigned(nch_all), 1024, smem, s>>>(static_cast<const int32_t*>(d_ids), d_offsets, id_base, V,
-                                                            C, int(Cq), planes, irr, err);
+                                                            C, int(Cq), planes, irr, num_ids, err);
         SE_CHECK_LAUNCH();
     } else {
         if (id_bytes == 4)
-            launch_positions(static_cast<const int32_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, err, s);
+            launch_positions(static_cast<const int32_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, num_ids, err,
+                             s);
         else if (id_bytes == 2)
-            launch_positions(static_cast<const uint16_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, err, s);
+            launch_positions(static_cast<const uint16_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, num_ids, err,
+                             s);
         else
-            launch_positions(static_cast<const uint8_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, err, s);
+            launch_positions(static_cast<const uint8_t*>(d_ids), d_offsets, id_base, V, C, Cq, pos, irr, num_ids, err,
+                             s);
         SE_CHECK_LAUNCH();
         K.pack<<<dim3(unsigned(nch_all), unsigned((Cq + 255) / 256)), 256, 0, s>>>(pos, V, Cq, planes);
         SE_CHECK_LAUNCH();
@@ -595,9 +618,10 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     // over all voters / splits + its output). Split outputs are atomic adds, dearer than the
     // plain stores of an unsplit launch. Costs in microseconds, measured on B200: counting
     // 0.15 per 32-voter chunk and plane-plus-two, output 12 (atomic) or 3 (stores) per tile.
-    // Take the cheapest split count (the smallest within 1 %), keeping at least 32 chunks (1024
-    // voters) per range. With few tiles and many voters this fills the SMs (C = 1024, 2^16
-    // voters: 36 tiles x 37 splits = 9 full waves on 148 SMs); with many tiles it stays 1.
+    // Take the cheapest split count (the smallest within 1 %), keeping at least 2 chunks (64
+    // voters) per range. With few tiles this fills the SMs (C = 1024, 2^16 voters: 36 tiles x 37
+    // splits = 9 full waves on 148 SMs; C = 128, 2000 voters: the one tile in 31 ranges); with many
+    // tiles it stays 1.
     // Then, unsplit, the last partial wave's tiles alone may be split the same way, when that
     // is cheaper than a whole wave for them (C = 4096, 4096 voters: 84 tiles in 3 ranges each;
     // C = 8192: 8 tiles in 4).
@@ -605,7 +629,7 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     SE_CUDA_TRY(cudaGetDevice(&dev));
     SE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t chunks = (V + kVC - 1) / kVC;
-    const int64_t max_splits = std::min<int64_t>(std::max<int64_t>(1, chunks / 32), 256);
+    const int64_t max_splits = std::min<int64_t>(std::max<int64_t>(1, chunks / 2), 256);
     const double full_us = 0.15 * double(chunks) * double(B + 2);
     int splits = 1;
     double best = 0.0;
@@ -672,6 +696,7 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     uint32_t code = 0;
     SE_CUDA_TRY(cudaMemcpyAsync(&code, err, 4, cudaMemcpyDeviceToHost, s));
     SE_CUDA_TRY(cudaStreamSynchronize(s));
+    SE_REQUIRE(code != kErrOffsets, SE_ERR_INVALID, "offsets must start at 0, never decrease and end at len(ids)");
     SE_REQUIRE(code != kErrRange, SE_ERR_DEVICE, "a ballot names a candidate outside [0, %d)", C);
     SE_REQUIRE(code == 0, SE_ERR_DEVICE, "tally kernel reported device error %u (TMA wait timed out)", code);
     return SE_OK;
@@ -683,6 +708,15 @@ extern "C" se_status_t se_tally(const int32_t* d_ids, const int64_t* d_offsets, 
     clear_error();
     SE_REQUIRE(V == 0 || d_offsets != nullptr, SE_ERR_INVALID, "null ballot pointer");
     return tally_impl(d_ids, 4, d_offsets, 0, V, C, 0u, d_out, ld_out, d_work, work_bytes, stream);
+}
+
+extern "C" se_status_t se_tally_checked(const int32_t* d_ids, int64_t num_ids, const int64_t* d_offsets, int64_t V,
+                                        int C, uint32_t* d_out, int64_t ld_out, void* d_work, int64_t work_bytes,
+                                        void* stream) {
+    clear_error();
+    SE_REQUIRE(V == 0 || d_offsets != nullptr, SE_ERR_INVALID, "null ballot pointer");
+    SE_REQUIRE(num_ids >= 0, SE_ERR_INVALID, "negative number of ids");
+    return tally_impl(d_ids, 4, d_offsets, 0, V, C, 0u, d_out, ld_out, d_work, work_bytes, stream, num_ids);
 }
 
 extern "C" se_status_t se_tally_enqueue(const int32_t* d_ids, const int64_t* d_offsets, int64_t V, int C,
