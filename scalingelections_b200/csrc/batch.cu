@@ -840,6 +840,18 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
     const int occ16 = occupancy<16>(), occ32 = occupancy<32>(), occ16w = occupancy<16, 4>();
     SE_REQUIRE(occ16 >= 1 && occ32 >= 1 && occ16w >= 1, SE_ERR_CUDA, "batched closure kernel cannot be resident");
     SE_REQUIRE(ctas_per_sm >= 0, SE_ERR_INVALID, "ctas_per_sm must be >= 0");
+    // Two CTAs per SM finish a tile task every 12.6 us and SM, one CTA every 16 us, but a round of
+    // the largest election's chain (pivot, panels, its remainder) takes about 74 us with a second CTA
+    // beside it and 51 us without. So a batch whose tasks are few for its chain takes one CTA per
+    // SM: tasks * 3.4 us / SMs < rounds * 23 us (a small election's task is about 12 us the shorter
+    // for a second CTA, a 32-bit tile's about 7). One B200, 20 elections up to C = 2048: 1799 -> 1590
+    // us, up to C = 700: 536 -> 410 us; 4096 elections (1.16 M tasks, 16 rounds) stay at two.
+    if (ctas_per_sm == 0 && Rmax > 1) {
+        const double nsmall = double(n) - double(big.size());
+        const double gain = 12.0 * nsmall + 3.4 * (double(P.ntasks[0]) + double(P.ntasks[2]) - nsmall) +
+                            7.0 * double(P.ntasks[1]);
+        if (gain < double(Rmax) * 23.0 * double(sms)) ctas_per_sm = 1;
+    }
     const int per16 = ctas_per_sm > 0 ? std::min(occ16, ctas_per_sm) : occ16;
     const int per32 = ctas_per_sm > 0 ? std::min(occ32, ctas_per_sm) : occ32;
     const int per16w = ctas_per_sm > 0 ? std::min(occ16w, ctas_per_sm) : occ16w;
