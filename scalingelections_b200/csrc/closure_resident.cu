@@ -1,11 +1,11 @@
 // One-launch closure of a small matrix: the whole working matrix stays in registers.
 //
-// Up to C = 2048 (16-bit lanes) the padded matrix fits the register files of the GPU's SMs. The
+// Up to C = 1536 (16-bit lanes) the padded matrix fits the register files of the GPU's SMs with room. The
 // schedules of closure.cu keep it in L2 and run two launches per 128-pivot round; at these sizes
 // their time is the serial chain of a round (close the 128-pivot tile, the panels, the next
 // diagonal tile, two launches), about 52 us a round whatever the size, with most SMs idle. Here
 //   * one cooperative launch runs the defeat init, every round and the widened output;
-//   * each CTA (one per SM) owns a row of CB blocks of 64 x 64 cells and keeps them in registers;
+//   * each CTA (one or two per SM) owns a row of CB blocks of 64 x 64 cells and keeps them in registers;
 //   * a round has 32 pivots, half a block: what is serial in a round (closing a 32 x 32 piece, its
 //     product with the next row and column pieces, the next diagonal piece) is short;
 //   * there is no barrier between rounds. Round k's panel blocks A[k][i] (its pivot columns in
@@ -58,7 +58,6 @@ using closure::ld4;
 using closure::st4;
 
 constexpr uint64_t kWaitNs = 2000000000ull;  // one wait
-constexpr int kStages = 4;
 constexpr int kP = 32;               // pivots per round
 constexpr int kNT = 256;             // compute threads
 constexpr int kThreads = kNT + 96;  // and the helper warps: the producer and two publishers
@@ -379,7 +378,7 @@ __device__ __forceinline__ void load_defeats(uint32_t (&c)[geo<LB>::QR][geo<LB>:
 // Dynamic shared memory: the stages' A and B slots, D of the last even and odd round in both forms,
 // each pair's piece of the diagonal block's work in both forms, a received side piece in both forms,
 // and the closing's staging rows.
-template <int LB, int CB> struct smem_layout {
+template <int LB, int CB, int kStages> struct smem_layout {
     using G = geo<LB>;
     static constexpr int STAGE = G::A_WORDS + CB * G::B_WORDS;
     static constexpr int DT = kStages * STAGE;
@@ -393,10 +392,10 @@ template <int LB, int CB> struct smem_layout {
     static constexpr int BYTES = WORDS * 4;
 };
 
-template <int LB, int CB, int OCC>
+template <int LB, int CB, int OCC, int kStages>
 __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_constant__ Params P) {
     using G = geo<LB>;
-    using SL = smem_layout<LB, CB>;
+    using SL = smem_layout<LB, CB, kStages>;
     constexpr int QR = G::QR, QC = G::QC, WH = G::WPB / 2;
     constexpr bool kEarly = CB == 1;  // diagonal() runs two rounds ahead
     extern __shared__ __align__(1024) uint32_t smem[];
@@ -896,22 +895,25 @@ struct Shape {
     int smem;
 };
 
-template <int LB, int CB, int OCC> Shape shape() {
-    return {CB, OCC, reinterpret_cast<const void*>(resident_kernel<LB, CB, OCC>), smem_layout<LB, CB>::BYTES};
+template <int LB, int CB, int OCC, int ST> Shape shape() {
+    return {CB, OCC, reinterpret_cast<const void*>(resident_kernel<LB, CB, OCC, ST>), smem_layout<LB, CB, ST>::BYTES};
 }
 
 // Shapes from the smallest tile to the largest; a matrix takes the first whose CTAs all fit the GPU.
-// Fewer blocks per CTA leave a panel less work between two steps of the chain. One B200, se_closure
-// with 16-bit lanes, us (blocks per CTA x CTAs per SM; last the launches of closure.cu):
-//   C = 768    1x1 159   1x2 172   2x1 218   2x2 253   launches 329
-//   C = 1024             1x2 225   2x1 282   2x2 310   launches 429
-//   C = 1344                       3x1 442   2x2 443   launches 612
-//   C = 1500                       4x1 586   2x2 497   launches 694
-// Two CTAs per SM take no more than 80 registers a thread, and in 32-bit lanes their slots do not
-// fit; there 3 blocks per CTA end at C = 1344, beyond which the launches are the faster form.
+// Fewer blocks per CTA leave a panel less work between two steps of the chain. One B200, se_closure,
+// us (blocks per CTA x CTAs per SM; last the launches of closure.cu):
+//   16-bit lanes   C = 768    1x1 159   1x2 172   2x1 218   2x2 253   launches 329
+//                  C = 1024             1x2 230   2x1 282   2x2 309   launches 429
+//                  C = 1344                       3x1 442   2x2 433   launches 612
+//                  C = 1500             4x1 586   2x2 487   3x2 596   launches 694
+//                  C = 2048                       3x2 966   4x2 1028  launches 950: not taken
+//   32-bit lanes   C = 1024             1x2 329   2x1 373             launches 593
+//                  C = 1344                       3x1 610   2x2 820   launches 777
+//                  C = 1500                       4x1 879             launches 866: not taken
+// Two CTAs per SM take no more than 80 registers a thread, and in 32-bit lanes three stages.
 const Shape* shapes(int lane_bits, int* n) {
-    static const Shape s16[] = {shape<16, 1, 1>(), shape<16, 1, 2>(), shape<16, 2, 2>()};
-    static const Shape s32[] = {shape<32, 1, 1>(), shape<32, 2, 1>(), shape<32, 3, 1>()};
+    static const Shape s16[] = {shape<16, 1, 1, 4>(), shape<16, 1, 2, 4>(), shape<16, 2, 2, 4>()};
+    static const Shape s32[] = {shape<32, 1, 1, 4>(), shape<32, 1, 2, 3>(), shape<32, 3, 1, 4>()};
     *n = 3;
     return lane_bits == 16 ? s16 : s32;
 }

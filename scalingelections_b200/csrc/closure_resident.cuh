@@ -11,8 +11,8 @@ namespace resident {
 
 constexpr int kB = 64;  // block edge, in cells
 
-// Largest C whose matrix fits the register files of 148 SMs: 32 x 4 tiles of 64 x 512 cells in
-// 16-bit lanes, 24 x 6 tiles of 64 x 256 cells in 32-bit lanes.
+// Largest C whose tiles all fit 148 SMs at once: 24 x 12 tiles of 64 x 128 cells, two per SM, in
+// 16-bit lanes; 21 x 7 tiles of 64 x 192 cells in 32-bit lanes.
 constexpr int max_candidates(int lane_bits) { return lane_bits == 16 ? 1536 : 1344; }
 
 // Workspace bytes of the resident closure, 0 where it does not apply.
