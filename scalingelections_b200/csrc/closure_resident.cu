@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
                             ok = false;
                             break;
                         }
-                        __nanosleep(40);  // the compute warps need the issue slots more
+                        __nanosleep(200);  // the compute warps need the issue slots (1 % of a call against 40 ns)
                     }
                     if (!ok) {
                         raise_device_error(P.words + kWordErr, kErrTmaTimeout);
