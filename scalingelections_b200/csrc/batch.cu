@@ -6,7 +6,8 @@
 //   SMALL      an election with C <= 128, whole in one CTA: defeat init from d, closure over
 //              its C pivots in registers, u32 output, wins and ranking. Nothing in HBM but d
 //              and the outputs.
-//   PIVOT k    close the pivot tile (k, k) of a larger election in registers; emit dT.
+//   PIVOT 0    close the pivot tile (0, 0) of a larger election in registers; emit dT. The task of
+//              remainder tile (k + 1, k + 1) closes it as the next pivot right after its update.
 //   ROW k, j   pivot-row panel tile (k, j)       = max(P, D (x) P)
 //   COL k, i   pivot-column panel tile (i, k)    = max(P, P (x) D); emit AT (transposed).
 //   REM k,i,j  remainder tile (i, j)             = max(S, AT (x) S[k][j])
@@ -14,12 +15,14 @@
 //
 // Scheduling: one persistent grid (every CTA resident) pulls tasks from a queue with an atomic
 // counter. The queue is ordered so that every task comes after the tasks it depends on:
-// round-major across elections (all pivots of round k, then all panels, then all remainders,
-// largest elections first), then the SMALL tasks, which fill the tail. A task waits (thread 0,
-// bounded by %globaltimer) on its election's per-round counters:
-//   PIVOT k   needs REM k-1 complete ((R-1)^2 tiles)
-//   ROW/COL k needs PIVOT k
+// round-major across elections (the pivots of round 0; then per round all panels, then all
+// remainders with the next pivot's tile first, largest elections first), then the SMALL tasks, which
+// fill the tail. A task waits (thread 0, bounded by %globaltimer) on its election's per-round counters:
+//   ROW/COL 0 needs PIVOT 0
+//   ROW/COL k needs REM k-1 complete ((R-1)^2 tiles, the next pivot's closing included)
 //   REM k     needs all 2(R-1) panels of round k
+// With a PIVOT task of its own in every round, a batch with few tasks for its chain waited for it alone:
+// 20 elections up to C = 2048 took 1594 us on one B200, now 1418 us.
 // Because a task's prerequisites were dequeued earlier by CTAs that are running, and those only
 // wait on even earlier tasks, the schedule cannot deadlock. A wait that times out sets the
 // error word and an abort flag that makes every CTA drain the queue and exit.
@@ -57,16 +60,13 @@ struct Header {
 };
 
 // The counter a task of election E waits for and the value it must reach; false for a task
-// with no dependency (SMALL, and PIVOT 0).
+// with no dependency (SMALL and PIVOT).
 __device__ __forceinline__ bool task_dependency(const Elec& E, uint32_t type, uint32_t k, const uint32_t*& ctr,
                                                 uint32_t& target) {
     const uint32_t R = uint32_t(E.R);
-    if (type == kPivot && k > 0) {
-        ctr = &E.counters[2 * R + k - 1];
-        target = (R - 1) * (R - 1);
-    } else if (type == kRow || type == kCol) {
-        ctr = &E.counters[k];
-        target = 1u;
+    if (type == kRow || type == kCol) {
+        ctr = k ? &E.counters[2 * R + k - 1] : &E.counters[0];
+        target = k ? (R - 1) * (R - 1) : 1u;
     } else if (type == kRem) {
         ctr = &E.counters[R + k];
         target = 2u * (R - 1);
@@ -158,11 +158,17 @@ __global__ void __launch_bounds__(tile_threads<LB, NQ>(), NQ == 4 ? 2 : 1)
         if (type == kSmall) {
             if constexpr (NQ == 8) run_small<LB>(E, smem, rowbuf, colbuf, s_wins, &hdr->err);
             else ok = false;  // the host never queues one here
-        } else if (type == kPivot) {
-            run_pivot<LB, NQ>(E, int(k), rowbuf, colbuf);
         } else {
-            const int kind = type == kRow ? kTileRow : (type == kCol ? kTileCol : kTileRem);
-            ok = run_tile<LB, true, NQ>(E, &E, kind, int(k), int(i), int(j), smem, bars, par_a, par_b);
+            int pivot = type == kPivot ? int(k) : -1;
+            if (type != kPivot) {
+                const int kind = type == kRow ? kTileRow : (type == kCol ? kTileCol : kTileRem);
+                ok = run_tile<LB, true, NQ>(E, &E, kind, int(k), int(i), int(j), smem, bars, par_a, par_b);
+                if (type == kRem && i == k + 1 && j == k + 1) {  // the next pivot's tile
+                    ok = __syncthreads_and(ok);                  // its stores are visible to the whole CTA
+                    if (ok) pivot = int(k) + 1;
+                }
+            }
+            if (pivot >= 0) run_pivot<LB, NQ>(E, pivot, rowbuf, colbuf);
         }
         __threadfence();
         __syncthreads();
@@ -589,7 +595,7 @@ se_status_t size_batch(int n, const se_election_t* el, Sizes& z) {
         z.dt_off[e] = off;
         off = align256(off + int64_t(kT) * kT * 4);
         const uint64_t R = uint64_t(z.R[e]);
-        z.ntasks[z.queue[e]] += uint32_t(R * R * R);
+        z.ntasks[z.queue[e]] += uint32_t(R * R * R - (R - 1));  // one pivot task, not R
         const int64_t nt = z.Cp[e] / kPT;
         z.pairs += nt * (nt + 1) / 2;
     }
@@ -757,8 +763,8 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
     if (order == 1)  // small elections first
         for (int l = 0; l < 2; ++l) q[l].insert(q[l].end(), small[l].begin(), small[l].end());
     for (int k = 0; k < Rmax; ++k) {
-        for (int e : order_big)
-            if (host[e].R > k) q[z.queue[e]].push_back(pack_task(e, kPivot, k, k, k));
+        if (k == 0)
+            for (int e : order_big) q[z.queue[e]].push_back(pack_task(e, kPivot, 0, 0, 0));
         for (int e : order_big)
             if (host[e].R > k) {
                 auto& Q = q[z.queue[e]];
@@ -771,10 +777,11 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
         for (int e : order_big)
             if (host[e].R > k) {
                 auto& Q = q[z.queue[e]];
+                if (k + 1 < host[e].R) Q.push_back(pack_task(e, kRem, k, k + 1, k + 1));
                 for (int i = 0; i < host[e].R; ++i)
                     if (i != k)
                         for (int j = 0; j < host[e].R; ++j)
-                            if (j != k) Q.push_back(pack_task(e, kRem, k, i, j));
+                            if (j != k && !(i == k + 1 && j == k + 1)) Q.push_back(pack_task(e, kRem, k, i, j));
             }
     }
     if (order != 1)
@@ -841,16 +848,17 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
     SE_REQUIRE(occ16 >= 1 && occ32 >= 1 && occ16w >= 1, SE_ERR_CUDA, "batched closure kernel cannot be resident");
     SE_REQUIRE(ctas_per_sm >= 0, SE_ERR_INVALID, "ctas_per_sm must be >= 0");
     // Two CTAs per SM finish a tile task every 12.6 us and SM, one CTA every 16 us, but a round of
-    // the largest election's chain (pivot, panels, its remainder) takes about 74 us with a second CTA
-    // beside it and 51 us without. So a batch whose tasks are few for its chain takes one CTA per
-    // SM: tasks * 3.4 us / SMs < rounds * 23 us (a small election's task is about 12 us the shorter
-    // for a second CTA, a 32-bit tile's about 7). One B200, 20 elections up to C = 2048: 1799 -> 1590
-    // us, up to C = 700: 536 -> 410 us; 4096 elections (1.16 M tasks, 16 rounds) stay at two.
+    // the largest election's chain (panels, its first remainder tile with the next pivot) takes
+    // longer beside a second CTA. So a batch whose tasks are few for its chain takes one CTA per SM:
+    // tasks * 3.4 us / SMs < rounds * 17 us, with the 17 fitted (a small election's task is about
+    // 12 us the shorter for a second CTA, a 32-bit tile's about 7). One B200, us with one / two CTAs
+    // per SM, sizes log-uniform: 20 elections up to C = 2048 1442 / 1567, 40 1938 / 1895, 100 3749 /
+    // 3374; 20 up to C = 700 400 / 490, 100 447 / 524, 300 818 / 820; 1000 up to C = 300 560 / 494.
     if (ctas_per_sm == 0 && Rmax > 1) {
         const double nsmall = double(n) - double(big.size());
         const double gain = 12.0 * nsmall + 3.4 * (double(P.ntasks[0]) + double(P.ntasks[2]) - nsmall) +
                             7.0 * double(P.ntasks[1]);
-        if (gain < double(Rmax) * 23.0 * double(sms)) ctas_per_sm = 1;
+        if (gain < double(Rmax) * 17.0 * double(sms)) ctas_per_sm = 1;
     }
     const int per16 = ctas_per_sm > 0 ? std::min(occ16, ctas_per_sm) : occ16;
     const int per32 = ctas_per_sm > 0 ? std::min(occ32, ctas_per_sm) : occ32;
