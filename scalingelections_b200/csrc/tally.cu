@@ -139,6 +139,31 @@ void launch_positions(const Id* ids, const int64_t* offsets, int64_t id_base, in
 // ------------------------------------------------------------------------------------------
 constexpr int kBitStages = 4;
 
+// Bit planes of 16 bits of 32 voters' places. On entry w[u] holds voter u's bits in its low half
+// and voter u + 16's in its high half; on return bit v of w[k] is bit k of voter v. Both halves
+// are transposed at once by swapping off-diagonal squares of 8, 4, 2 and 1 bits: about 130
+// instructions a word of 32 places (the rows past the last plane are dead code), against two per
+// voter and plane (640 at B = 10) when each bit is extracted and inserted by itself.
+__device__ __forceinline__ void transpose_places(uint32_t (&w)[16]) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const uint32_t a = w[u], b = w[u + 8];
+        w[u] = __byte_perm(a, b, 0x6240);
+        w[u + 8] = __byte_perm(a, b, 0x7351);
+    }
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1) {
+        const uint32_t m = d == 4 ? 0x0F0F0F0Fu : d == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            if (u & d) continue;
+            const uint32_t a = w[u], b = w[u + d];
+            w[u] = (a & m) | ((b << d) & ~m);
+            w[u + d] = ((a >> d) & m) | (b & ~m);
+        }
+    }
+}
+
 // planes[(ch * B + k) * Cq + c] for the chunks of voters [0, V); voters past V count as place 0.
 // B is a template parameter so that only B planes of bit work are done, in registers.
 template <int B>
@@ -154,11 +179,14 @@ __global__ void __launch_bounds__(256)
         p[v] = voter < V ? uint32_t(pos[voter * Cq + c]) : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < B; ++k) {
-        uint32_t w = 0u;
+    for (int k0 = 0; k0 < B; k0 += 16) {
+        uint32_t w[16];
 #pragma unroll
-        for (int v = 0; v < 32; ++v) w |= ((p[v] >> k) & 1u) << v;
-        planes[(ch * B + k) * Cq + c] = w;
+        for (int u = 0; u < 16; ++u) w[u] = __byte_perm(p[u], p[u + 16], k0 ? 0x7632 : 0x5410);
+        transpose_places(w);
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (k0 + k < B) planes[(ch * B + k0 + k) * Cq + c] = w[k];
     }
 }
 
@@ -171,7 +199,7 @@ constexpr int kFusedMaxCq = 2048;
 inline size_t fused_smem(int64_t Cq) { return size_t(32) * size_t(Cq + 2) * 2; }
 
 template <typename Id, int B>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(1024, 2)
     places_planes_kernel(const Id* __restrict__ ids, const int64_t* __restrict__ offsets, int64_t id_base,
                          int64_t V, int C, int Cq, uint32_t* __restrict__ planes, Irregular irr, int64_t num_ids,
                          uint32_t* __restrict__ err) {
@@ -197,16 +225,12 @@ __global__ void __launch_bounds__(1024)
     }
     __syncthreads();
     for (int c = threadIdx.x; c < Cq; c += blockDim.x) {
-        uint32_t p[32];
+        uint32_t w[16];
 #pragma unroll
-        for (int u = 0; u < 32; ++u) p[u] = rows[u * pitch + c];
+        for (int u = 0; u < 16; ++u) w[u] = rows[u * pitch + c] | uint32_t(rows[(u + 16) * pitch + c]) << 16;
+        transpose_places(w);
 #pragma unroll
-        for (int k = 0; k < B; ++k) {
-            uint32_t word = 0u;
-#pragma unroll
-            for (int u = 0; u < 32; ++u) word |= ((p[u] >> k) & 1u) << u;
-            planes[(ch * B + k) * int64_t(Cq) + c] = word;
-        }
+        for (int k = 0; k < B; ++k) planes[(ch * B + k) * int64_t(Cq) + c] = w[k];
     }
 }
 
