@@ -18,8 +18,8 @@
 // complement V - d[i][j]. irregular_kernel then adds its pairs exactly as the reference does,
 // diagonal included, with atomics.
 // For C < 2048, places_planes_kernel does both in one pass and keeps the places in shared
-// memory. Kernel 3 (count_bits_kernel, one CTA per upper tile) streams the planes of the two
-// 128-candidate strips into shared memory with TMA and counts per 8 x 8 register micro-tile
+// memory. Kernel 3 (count_bits_kernel, one CTA per SM) streams the planes of each upper tile's two
+// 128-candidate strips into shared memory with TMA and counts per 8 x 4 register micro-tile
 // with a bit-serial borrow chain (one lop3 per plane) and a popc per 32 voters.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -242,46 +242,72 @@ __device__ __forceinline__ uint32_t borrow_step(uint32_t a, uint32_t b, uint32_t
 
 inline size_t bits_smem(int B) { return size_t(kBitStages) * 2 * B * kTile * 4 + kBitStages * 8; }
 
-// How the count's CTAs map to (upper tile, voter range). The first head_ctas CTAs take tiles
-// 0 .. head_ctas / splits - 1, each cut into `splits` voter ranges; the rest take the remaining
-// tiles (the launch's last, partial wave), each cut into tail_splits ranges, so that the tail
-// does not hold a whole wave's time for a few tiles.
+// How the count's CTAs share the work. The tiles are ordered with the n1 = R (R - 1) / 2 tiles
+// above the diagonal first, row by row, then the R diagonal tiles. CTA b of the G (one per SM)
+// takes the whole tiles b, b + G, .. of the first `rounds` * G, all above the diagonal. The rest
+// is laid end to end as a line of (tile, 32-voter chunk) units and cut into G equal ranges, where
+// a unit above the diagonal weighs 5 and a diagonal one 4 (count_bits_kernel leaves out warps
+// there; the count of C = 1000, V = 60000 takes 724 us so, 755 with 4 and 3, 769 with equal
+// weights). A range ends anywhere inside a tile; such a tile's counts arrive as atomic adds.
+// `whole` moves the ends to tile ends. So no SM waits for a last partial wave, and a CTA has at
+// most two split tiles to add, however many voters there are.
 struct CountSplit {
-    int64_t head_ctas;
-    int splits;
-    int tail_splits;
+    int64_t rounds;
+    bool whole;
 };
 
-// Upper tile t (row by row: row I holds tiles (I, I) .. (I, R - 1)).
-__device__ __forceinline__ void upper_tile(int64_t t, int R, int& I, int& J) {
-    I = 0;
-    while (t >= R - I) {
-        t -= R - I;
-        ++I;
+__host__ __device__ inline int64_t tiles_above(int R) { return int64_t(R) * (R - 1) / 2; }
+
+// Tile t of that order.
+__device__ __forceinline__ void count_tile(int64_t t, int R, int& I, int& J) {
+    const int64_t n1 = tiles_above(R);
+    if (t < n1) {
+        upper_pair(t, R - 1, I, J);
+        ++J;
+    } else {
+        I = J = int(t - n1);
     }
-    J = I + int(t);
 }
 
-// Zeroes upper tile first + blockIdx.x and its mirror (J, I), row by row: the tiles whose counts
-// arrive as atomic adds from several voter ranges.
+// First unit of CTA b's range of the line (b = G: its end).
+__device__ __forceinline__ int64_t range_start(const CountSplit& sp, int R, int64_t chunks, int64_t b, int64_t G) {
+    const int64_t above = tiles_above(R) - sp.rounds * G;  // tiles of the line above the diagonal
+    if (sp.whole) return (above + R) * b / G * chunks;
+    const int64_t x = (5 * above + 4 * R) * chunks * b / G;
+    return x <= 5 * above * chunks ? x / 5 : above * chunks + (x - 5 * above * chunks) / 4;
+}
+
+// Zeroes the tiles that range ends cut, and their mirrors: blocks (b, *) look at the start of range
+// b + 1 of G = gridDim.x + 1, and leave a tile that an earlier range's start cuts to that one's.
+// Each of the gridDim.y blocks of a tile takes its share of the rows.
+constexpr int kZeroParts = 8;
+
 __global__ void __launch_bounds__(256)
-    zero_tiles_kernel(uint32_t* __restrict__ out, int64_t ld_out, int C, int R, int64_t first) {
+    zero_tiles_kernel(uint32_t* __restrict__ out, int64_t ld_out, int C, int R, int64_t chunks, CountSplit sp) {
+    const int64_t b = int64_t(blockIdx.x) + 1, G = int64_t(gridDim.x) + 1;
+    const int64_t u = range_start(sp, R, chunks, b, G), t = u / chunks;
+    if (u % chunks == 0) return;
+    const int64_t before = range_start(sp, R, chunks, b - 1, G);
+    if (before / chunks == t && before % chunks != 0) return;
     int I, J;
-    upper_tile(first + blockIdx.x, R, I, J);
-    for (int e = threadIdx.x; e < kTile * kTile; e += 256) {
+    count_tile(sp.rounds * G + t, R, I, J);
+    for (int e = blockIdx.y * 256 + threadIdx.x; e < kTile * kTile; e += gridDim.y * 256) {
         const int r = e / kTile, c = e % kTile;
         if (I * kTile + r < C && J * kTile + c < C) out[int64_t(I * kTile + r) * ld_out + J * kTile + c] = 0u;
-        if (J * kTile + r < C && I * kTile + c < C) out[int64_t(J * kTile + r) * ld_out + I * kTile + c] = 0u;
+        if (I != J && J * kTile + r < C && I * kTile + c < C) out[int64_t(J * kTile + r) * ld_out + I * kTile + c] = 0u;
     }
 }
 
-// Counting over one upper tile (I <= J): d[I][J] and, for I < J, d[J][I] = V - d[I][J]. One
-// CTA per tile (and voter range): the two 128-candidate plane strips of each 32-voter chunk
-// are staged by TMA (box {128, B}) through a 4-stage ring. With splits > 1 the voters are cut
-// into `splits` ranges of whole chunks, one CTA per (tile, range), and each CTA adds its
-// range's counts (and, below the diagonal, the range's voters minus them) to out with atomics:
-// exact, since every count is an integer, and it keeps the grid full when there are few tiles
-// and many voters.
+// Counting over upper tiles (I <= J): d[I][J] and, for I < J, d[J][I] = V - d[I][J]. One CTA per
+// SM works through its tiles (CountSplit): the two 128-candidate plane strips of each 32-voter
+// chunk are staged by TMA (box {128, B}) through a 4-stage ring that runs on across its tiles, so
+// the next tile's first chunks arrive while this one's counts go out. The ALU pipe is the bound
+// (87 % active); before the tiles were shared out evenly, each CTA took one tile or a fixed share
+// of one, and the last wave, the many small shares' adds and the full diagonal tiles cost the
+// rest.
+// A diagonal tile's mirror image lies in itself: its 6 warps (of 16, one 32 x 32 block each) below
+// the diagonal count nothing, and the warps above write both cells. The blocks are dealt to the
+// warps such that each scheduler (warp mod 4) keeps at most 3 of its 4.
 // B (the planes per chunk) is a template parameter: the plane loop unrolls fully.
 template <int B>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -295,148 +321,170 @@ __global__ void __launch_bounds__(kThreads, 1)
     constexpr uint32_t stage_words = uint32_t(B) * kTile;
     constexpr uint32_t stage_bytes = 2u * stage_words * 4u;
 
-    int64_t t;
-    int split, splits;
-    if (int64_t(blockIdx.x) < sp.head_ctas) {
-        t = blockIdx.x / sp.splits, split = int(blockIdx.x % sp.splits), splits = sp.splits;
-    } else {
-        const int64_t b = int64_t(blockIdx.x) - sp.head_ctas;
-        t = sp.head_ctas / sp.splits + b / sp.tail_splits, split = int(b % sp.tail_splits), splits = sp.tail_splits;
-    }
-    int I, J;
-    upper_tile(t, R, I, J);
-    const int total_ch = int((V + kVC - 1) / kVC);
-    const int per = (total_ch + splits - 1) / splits;
-    const int ch0 = split * per < total_ch ? split * per : total_ch;
-    const int ch1 = ch0 + per < total_ch ? ch0 + per : total_ch;
-    const int nch = ch1 - ch0;
-    const int64_t vlo = int64_t(ch0) * kVC, vhi = int64_t(ch1) * kVC < V ? int64_t(ch1) * kVC : V;
+    const int64_t G = gridDim.x, cta = blockIdx.x;
+    const int chunks = int((V + kVC - 1) / kVC);
+    const int64_t start = range_start(sp, R, chunks, cta, G);
+    const int64_t in_rounds = sp.rounds * chunks;  // units in whole-tile rounds
+    const int64_t units = in_rounds + range_start(sp, R, chunks, cta + 1, G) - start;
+    // Unit n of this CTA: its tile and chunk.
+    auto locate = [&](int64_t n, int& I, int& J, int& ch) {
+        const int64_t u = n < in_rounds ? n : start + (n - in_rounds);
+        const int64_t q = u / chunks;
+        ch = int(u - q * chunks);
+        count_tile(n < in_rounds ? cta + G * q : sp.rounds * G + q, R, I, J);
+    };
+    auto load = [&](int s, int I, int J, int ch) {
+        mbar_arrive_expect_tx(&bars[s], stage_bytes);
+        tma_load_2d(sI + s * stage_words, &mapPl, &bars[s], I * kTile, ch * B);
+        tma_load_2d(sJ + s * stage_words, &mapPl, &bars[s], J * kTile, ch * B);
+    };
 
     // done[s]: warps finished with stage s's current chunk. The last of them refills the stage
     // (see the end of the chunk loop), so no warp waits for another except on the data.
     __shared__ uint32_t done[kBitStages];
-    __shared__ uint32_t irr_in_range;  // irregular ballots among this CTA's voters
     if (threadIdx.x < kBitStages) done[threadIdx.x] = 0u;
-    if (threadIdx.x < 32) {
-        uint32_t n = 0u;
-        for (int c = ch0 + int(threadIdx.x); c < ch1; c += 32) n += irr_chunk[c];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-        if (threadIdx.x == 0) irr_in_range = n;
-    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kBitStages; ++s) mbar_init(&bars[s], 1);
         fence_barrier_init();
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kBitStages && s < nch; ++s) {
-            mbar_arrive_expect_tx(&bars[s], stage_bytes);
-            tma_load_2d(sI + s * stage_words, &mapPl, &bars[s], I * kTile, (ch0 + s) * B);
-            tma_load_2d(sJ + s * stage_words, &mapPl, &bars[s], J * kTile, (ch0 + s) * B);
+        for (int s = 0; s < kBitStages && s < units; ++s) {
+            int I, J, ch;
+            locate(s, I, J, ch);
+            load(s, I, J, ch);
         }
     }
     // 16 warps: rows row0..row0+7 and columns col0..col0+3 of the tile per thread. A warp's 8
     // column groups read 128 contiguous bytes of a plane; its 4 row groups read 4 x 32 bytes.
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = (warp & 3) * 32 + (lane >> 3) * 8;
-    const int col0 = (warp >> 2) * 32 + (lane & 7) * 4;
-    uint32_t acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0u;
+    const int cb = warp >> 2, rb = ((warp & 3) + (cb == 1 || cb == 2 ? 3 : 0)) & 3;
+    const int row0 = rb * 32 + (lane >> 3) * 8;
+    const int col0 = cb * 32 + (lane & 7) * 4;
 
+    const bool wide = !accumulate && ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     bool ok = true;
+    int s = 0;           // the next unit's stage and its phase
+    uint32_t phase = 0;
+    int64_t n = 0;       // the tile's first unit
 #pragma unroll 1
-    for (int ch = 0; ch < nch; ++ch) {
-        const int s = ch % kBitStages;
-        if (ok && !mbar_wait_bounded(&bars[s], uint32_t(ch / kBitStages) & 1u, kMaxPolls)) ok = false;
-        if (ok) {
-            const uint32_t* pI = sI + s * stage_words;
-            const uint32_t* pJ = sJ + s * stage_words;
-            uint32_t br[8][4];
+    while (n < units) {
+        int I, J, ch0;
+        locate(n, I, J, ch0);
+        const int ch1 = int(units - n < chunks - ch0 ? ch0 + (units - n) : chunks);
+        const bool counts = I != J || rb <= cb;
+        uint32_t acc[8][4];
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) br[r][q] = 0u;
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                uint32_t a[8], b[4];
-                const uint4 a0 = *reinterpret_cast<const uint4*>(pI + k * kTile + row0);
-                const uint4 a1 = *reinterpret_cast<const uint4*>(pI + k * kTile + row0 + 4);
-                const uint4 b0 = *reinterpret_cast<const uint4*>(pJ + k * kTile + col0);
-                a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w, a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
-                b[0] = b0.x, b[1] = b0.y, b[2] = b0.z, b[3] = b0.w;
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0u;
+#pragma unroll 1
+        for (int ch = ch0; ch < ch1; ++ch) {
+            if (ok && !mbar_wait_bounded(&bars[s], phase, kMaxPolls)) ok = false;
+            if (ok && counts) {
+                const uint32_t* pI = sI + s * stage_words;
+                const uint32_t* pJ = sJ + s * stage_words;
+                uint32_t br[8][4];
 #pragma unroll
                 for (int r = 0; r < 8; ++r)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) br[r][q] = borrow_step(a[r], b[q], br[r][q]);
+                    for (int q = 0; q < 4; ++q) br[r][q] = 0u;
+#pragma unroll
+                for (int k = 0; k < B; ++k) {
+                    uint32_t a[8], b[4];
+                    const uint4 a0 = *reinterpret_cast<const uint4*>(pI + k * kTile + row0);
+                    const uint4 a1 = *reinterpret_cast<const uint4*>(pI + k * kTile + row0 + 4);
+                    const uint4 b0 = *reinterpret_cast<const uint4*>(pJ + k * kTile + col0);
+                    a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w, a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
+                    b[0] = b0.x, b[1] = b0.y, b[2] = b0.z, b[3] = b0.w;
+#pragma unroll
+                    for (int r = 0; r < 8; ++r)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) br[r][q] = borrow_step(a[r], b[q], br[r][q]);
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) acc[r][q] += __popc(br[r][q]);
             }
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[r][q] += __popc(br[r][q]);
+            // This warp is done reading stage s. The last warp to get here refills it with unit
+            // kBitStages further on: its lane 0 has seen every other warp's count (and, through the warp
+            // barrier and the block fence, their reads of the stage come before the copy). Waiters
+            // on bars[s] acquire the reset of done[s] with the stage's next phase.
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence_block();
+                if (atomicAdd(&done[s], 1u) == uint32_t(kThreads / 32 - 1)) {
+                    done[s] = 0u;
+                    int nI = I, nJ = J, nch = ch + kBitStages;
+                    const int64_t next = n + (nch - ch0);
+                    if (ok && next < units) {
+                        if (nch >= ch1) locate(next, nI, nJ, nch);
+                        fence_proxy_async();
+                        load(s, nI, nJ, nch);
+                    }
+                }
+            }
+            if (++s == kBitStages) s = 0, phase ^= 1u;
         }
-        // This warp is done reading stage s. The last warp to get here refills it with chunk
-        // ch + kBitStages: its lane 0 has seen every other warp's count (and, through the warp
-        // barrier and the block fence, their reads of the stage come before the copy). Waiters
-        // on bars[s] acquire the reset of done[s] with the stage's next phase.
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence_block();
-            if (atomicAdd(&done[s], 1u) == uint32_t(kThreads / 32 - 1)) {
-                done[s] = 0u;
-                if (ok && ch + kBitStages < nch) {
-                    fence_proxy_async();
-                    mbar_arrive_expect_tx(&bars[s], stage_bytes);
-                    tma_load_2d(sI + s * stage_words, &mapPl, &bars[s], I * kTile, (ch0 + ch + kBitStages) * B);
-                    tma_load_2d(sJ + s * stage_words, &mapPl, &bars[s], J * kTile, (ch0 + ch + kBitStages) * B);
+        n += ch1 - ch0;
+        if (!ok) break;
+        if (!counts) continue;
+        // Voters with a permutation ballot: each of them is counted in exactly one of d[i][j] and
+        // d[j][i]. Irregular ballots (place 0 everywhere) are in neither and are added apart.
+        uint32_t irregular = 0u;
+        for (int c = ch0 + lane; c < ch1; c += 32) irregular += irr_chunk[c];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) irregular += __shfl_xor_sync(0xffffffffu, irregular, o);
+        const int64_t vlo = int64_t(ch0) * kVC, vhi = int64_t(ch1) * kVC < V ? int64_t(ch1) * kVC : V;
+        const uint32_t Vu = uint32_t(vhi - vlo) - irregular;
+        const bool split = ch1 - ch0 < chunks;
+        const bool mirror = I != J || rb != cb;
+        // A whole tile inside aligned rows goes out in 16-byte stores. Scalar ones cost the mirror
+        // image, whose rows lie along this thread's 8 rows, a sector per cell.
+        if (wide && !split && (J + 1) * kTile <= C) {
+            const int64_t i0 = int64_t(I) * kTile + row0, j0 = int64_t(J) * kTile + col0;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                uint32_t c[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) c[q] = i0 + r == j0 + q ? 0u : acc[r][q];
+                *reinterpret_cast<uint4*>(out + (i0 + r) * ld_out + j0) = make_uint4(c[0], c[1], c[2], c[3]);
+            }
+            if (!mirror) continue;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int r = 0; r < 8; r += 4)
+                    *reinterpret_cast<uint4*>(out + (j0 + q) * ld_out + i0 + r) =
+                        make_uint4(Vu - acc[r][q], Vu - acc[r + 1][q], Vu - acc[r + 2][q], Vu - acc[r + 3][q]);
+            continue;
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int i = I * kTile + row0 + r;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = J * kTile + col0 + q;
+                const uint32_t c = acc[r][q];
+                if (i < C && j < C) {
+                    uint32_t* ij = out + int64_t(i) * ld_out + j;
+                    uint32_t* ji = out + int64_t(j) * ld_out + i;
+                    if (split) {
+                        if (i != j) atomicAdd(ij, c);
+                        if (mirror) atomicAdd(ji, Vu - c);
+                    } else if (accumulate) {
+                        if (i != j) *ij += c;
+                        if (mirror) *ji += Vu - c;
+                    } else {
+                        *ij = i == j ? 0u : c;
+                        if (mirror) *ji = Vu - c;
+                    }
                 }
             }
         }
     }
-    if (!ok) {
-        raise_device_error(err, kErrTimeout);
-        return;
-    }
-    // Voters with a permutation ballot: each of them is counted in exactly one of d[i][j] and
-    // d[j][i]. Irregular ballots (place 0 everywhere) are in neither and are added apart.
-    const uint32_t Vu = uint32_t(vhi - vlo) - irr_in_range;
-    if (nch == 0) return;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int i = I * kTile + row0 + r;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = J * kTile + col0 + q;
-            const uint32_t n = acc[r][q];
-            if (i < C && j < C) {
-                uint32_t* ij = out + int64_t(i) * ld_out + j;
-                uint32_t* ji = out + int64_t(j) * ld_out + i;
-                if (splits > 1) {
-                    if (I != J) {
-                        atomicAdd(ij, n);
-                        atomicAdd(ji, Vu - n);
-                    } else if (i != j) {
-                        atomicAdd(ij, n);
-                    }
-                } else if (accumulate) {
-                    if (I != J) {
-                        *ij += n;
-                        *ji += Vu - n;
-                    } else if (i != j) {
-                        *ij += n;
-                    }
-                } else if (I == J) {
-                    *ij = i == j ? 0u : n;
-                } else {
-                    *ij = n;
-                    *ji = Vu - n;
-                }
-            }
-        }
-    }
+    if (!ok) raise_device_error(err, kErrTimeout);
 }
 
 // The pairs of the irregular ballots, as the reference counts them (py:46-48 over the ballot
@@ -636,59 +684,27 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     if (se_status_t st = se::closure::make_map(&map, planes, uint64_t(Cq), uint64_t(nch_all * B), uint64_t(Cq) * 4,
                                                kTile, uint32_t(B)))
         return st;
-    const int64_t tiles = int64_t(R) * (R + 1) / 2;
-    // Voter splits: each of the tiles x splits CTAs counts 1/splits of the voters, one CTA per
-    // SM at a time, so a launch takes ceil(tiles x splits / SMs) waves of (the tile's counting
-    // over all voters / splits + its output). Split outputs are atomic adds, dearer than the
-    // plain stores of an unsplit launch. Costs in microseconds, measured on B200: counting
-    // 0.15 per 32-voter chunk and plane-plus-two, output 12 (atomic) or 3 (stores) per tile.
-    // Take the cheapest split count (the smallest within 1 %), keeping at least 2 chunks (64
-    // voters) per range. With few tiles this fills the SMs (C = 1024, 2^16 voters: 36 tiles x 37
-    // splits = 9 full waves on 148 SMs; C = 128, 2000 voters: the one tile in 31 ranges); with many
-    // tiles it stays 1.
-    // Then, unsplit, the last partial wave's tiles alone may be split the same way, when that
-    // is cheaper than a whole wave for them (C = 4096, 4096 voters: 84 tiles in 3 ranges each;
-    // C = 8192: 8 tiles in 4).
+    // One CTA per SM (fewer when there are not two 32-voter chunks for each), all whole tiles that
+    // come out even, then the rest of the tiles cut into equal ranges (CountSplit). Cutting pays
+    // when the wait for the last whole tiles is longer than what it adds: an output by atomic adds
+    // at each end of a range and the zeroing before it. Costs in microseconds, measured on B200:
+    // counting 0.15 per 32-voter chunk and plane-plus-two, output 12 (atomic) or 3 (stores) per
+    // tile, zeroing 6.
     int sms = 0, dev = 0;
     SE_CUDA_TRY(cudaGetDevice(&dev));
     SE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t chunks = (V + kVC - 1) / kVC;
-    const int64_t max_splits = std::min<int64_t>(std::max<int64_t>(1, chunks / 2), 256);
+    const int64_t tiles = int64_t(R) * (R + 1) / 2;
+    const int64_t grid = std::min<int64_t>(sms, std::max<int64_t>(tiles, tiles * chunks / 2));
     const double full_us = 0.15 * double(chunks) * double(B + 2);
-    int splits = 1;
-    double best = 0.0;
-    for (int64_t sp = 1; sp <= max_splits; ++sp) {
-        const double waves = double((tiles * sp + sms - 1) / sms);
-        const double cost = waves * (full_us / double(sp) + (sp > 1 ? 12.0 : 3.0));
-        if (sp == 1 || cost < best * 0.99) {
-            best = cost;
-            splits = int(sp);
-        }
+    CountSplit layout{tiles_above(R) / grid, false};
+    const int64_t above = tiles_above(R) - layout.rounds * grid;
+    const double cut_us = (double(above) + 0.8 * R) / double(grid) * full_us + 2 * 12.0 + 6.0;
+    layout.whole = double((above + R + grid - 1) / grid) * (full_us + 3.0) <= cut_us;
+    if (!accumulate && !layout.whole && grid > 1) {
+        zero_tiles_kernel<<<dim3(unsigned(grid - 1), kZeroParts), 256, 0, s>>>(d_out, ld_out, C, R, chunks, layout);
+        SE_CHECK_LAUNCH();
     }
-    int64_t head = tiles;  // tiles in the head of the launch
-    int tail_splits = 1;
-    if (splits == 1 && tiles > sms && tiles % sms) {
-        const int64_t rem = tiles % sms;
-        double tail = full_us + 3.0;
-        for (int64_t sp = 2; sp <= std::min<int64_t>(max_splits, 8); ++sp) {
-            const double cost = double((rem * sp + sms - 1) / sms) * (full_us / double(sp) + 12.0);
-            if (cost < tail * 0.99) {
-                tail = cost;
-                tail_splits = int(sp);
-            }
-        }
-        if (tail_splits > 1) head = tiles - rem;
-    }
-    if (!accumulate) {
-        if (splits > 1) {
-            SE_CUDA_TRY(cudaMemset2DAsync(d_out, size_t(ld_out) * 4, 0, size_t(C) * 4, size_t(C), s));
-        } else if (tail_splits > 1) {
-            zero_tiles_kernel<<<unsigned(tiles - head), 256, 0, s>>>(d_out, ld_out, C, R, head);
-            SE_CHECK_LAUNCH();
-        }
-    }
-    const CountSplit layout{head * splits, splits, tail_splits};
-    const int64_t grid = head * splits + (tiles - head) * tail_splits;
     K.count<<<unsigned(grid), kThreads, bits_smem(B), s>>>(map, V, C, R, layout, d_out, ld_out, accumulate, irr.chunk,
                                                            err);
     SE_CHECK_LAUNCH();

@@ -37,6 +37,22 @@ def test_few_tiles(orc, V, C, ragged):
     assert np.array_equal(got, orc.tally(completed(rows, C), "positions"))
 
 
+@pytest.mark.parametrize("V", [31, 65, 290])
+@pytest.mark.parametrize("C", [1000, 2300, 2433])
+def test_whole_rounds_and_cut_tiles(orc, V, C):
+    """36 tiles, all cut; 171 and 190 above the diagonal, a round of whole tiles on 148 SMs and the
+    rest whole (few voters) or cut (many); ballots that repeat a candidate in whole and cut tiles."""
+    rows = ballots(V, C, False, seed=V + C)
+    ids, offs = to_device(rows)
+    got = api._to_host_u32(api.tally_device(ids, offs, C))
+    assert np.array_equal(got, orc.tally(np.stack(rows), "positions"))
+    for v in (0, V // 2, V - 1):
+        rows[v][1] = rows[v][0]
+    ids, offs = to_device(rows)
+    got = api._to_host_u32(api.tally_device(ids, offs, C))
+    assert np.array_equal(got, orc.tally(np.stack(rows), "scatter"))
+
+
 @pytest.mark.parametrize("C", [40, 2050])
 def test_bad_offsets_are_refused(C):
     rows = ballots(70, C, False, seed=C)
