@@ -108,7 +108,8 @@ SE_API se_status_t se_closure_check(const void* d_work, void* stream);
 /* Same as se_closure, and also fills phase_ms[4] with the summed device time of the four
  * kernel kinds (pivot tile, pivot-row panel, pivot-column panel, remainder) from CUDA events
  * recorded between the launches, and *launches with the number of kernels launched.
- * Synchronous. For profiling: the events add a little time between launches. */
+ * Synchronous. For profiling: the events add a little time between launches, and where
+ * se_closure would run the resident closure this runs the launches that it stands in for. */
 SE_API se_status_t se_closure_profiled(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t* d_out,
                                        int64_t ld_out, int lane_bits, int tile, void* d_work,
                                        int64_t work_bytes, void* stream, double* phase_ms, int* launches);
@@ -169,11 +170,23 @@ SE_API se_status_t se_closure_set_variant_table(const int* max_c, const int* mod
 
 /* The schedule (1 to 8) an se_closure call would run now for C candidates with lane_bits 16
  * or 32 and work_bytes of workspace; -1 for C < 1. Host-only. Where the automatic schedule
- * runs the resident closure, this is the schedule that it stands in for. */
+ * runs the resident closure (se_closure_resident), this is the schedule that it stands in for. */
 SE_API int se_closure_schedule(int C, int lane_bits, int64_t work_bytes);
 
-/* Number of kernels one se_closure call launches for C candidates in 16-bit lanes under the
- * current schedule (automatic lanes add at most one more; the resident closure is one launch). */
+/* 1 if the automatic schedule, as it is set now, tries the resident closure first for C
+ * candidates with lane_bits (0: its first attempt, in 16-bit lanes) and work_bytes of workspace;
+ * else 0. Host-only: it assumes a whole B200 and a stream that is not capturing. */
+SE_API int se_closure_resident(int C, int lane_bits, int64_t work_bytes);
+
+/* What the calling thread's last closure call (se_closure, se_closure_enqueue,
+ * se_closure_profiled, se_closure_noalloc) queued: schedule 1 to 8, SE_CLOSURE_RESIDENT, or 0 if
+ * it failed before it queued one or there was no call. */
+#define SE_CLOSURE_RESIDENT 9
+SE_API int se_closure_last_schedule(void);
+
+/* Number of kernels one se_closure call launches for C candidates in 16-bit lanes, with
+ * se_closure_workspace_bytes_flow() of workspace, under the current schedule (automatic lanes add
+ * at most one more): 1 where the resident closure runs. */
 SE_API int se_closure_launch_count(int C);
 
 /* Largest C that se_closure_noalloc accepts. */

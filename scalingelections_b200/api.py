@@ -170,14 +170,33 @@ def set_closure_mode(mode: int) -> None:
 BUILTIN_CLOSURE_VARIANTS = ((1024, 7), (4096, 8), (1 << 20, 6))
 
 
+CLOSURE_RESIDENT = 9  # last_closure_schedule(): the one-launch closure in registers
+
+
 def closure_schedule(num_candidates: int, lanes: int = LANES_U16, workspace_bytes: int | None = None) -> int:
     """The schedule (1 to 8) a closure of this size would run now (host-only query). The
-    workspace defaults to what strongest_paths_device allocates; -1 for no candidates."""
+    workspace defaults to what strongest_paths_device allocates; -1 for no candidates. Where
+    closure_is_resident says so, the one-launch closure stands in for it."""
     if int(num_candidates) < 1:
         return -1
     if workspace_bytes is None:
         workspace_bytes = closure_workspace_bytes(num_candidates, lanes, dataflow=True)
     return int(_lib.lib().se_closure_schedule(int(num_candidates), int(lanes), int(workspace_bytes)))
+
+
+def closure_is_resident(num_candidates: int, lanes: int = LANES_U16, workspace_bytes: int | None = None) -> bool:
+    """Whether the automatic schedule, as it is set now, tries the one-launch closure in registers
+    first (host-only query; a whole B200 and a stream outside a capture)."""
+    if int(num_candidates) < 1:
+        return False
+    if workspace_bytes is None:
+        workspace_bytes = closure_workspace_bytes(num_candidates, lanes, dataflow=True)
+    return bool(_lib.lib().se_closure_resident(int(num_candidates), int(lanes), int(workspace_bytes)))
+
+
+def last_closure_schedule() -> int:
+    """What this thread's last closure queued: schedule 1 to 8 or CLOSURE_RESIDENT (0: none)."""
+    return int(_lib.lib().se_closure_last_schedule())
 
 
 def set_closure_variants(table: Sequence[tuple[int, int]]) -> None:

@@ -779,6 +779,31 @@ int automatic_mode(int C) {
     return 1;
 }
 
+// The schedule (1 to 8) that `mode` comes to for a matrix of layout P and a workspace: where the
+// workspace or the number of rounds is too small for it, the automatic choice takes the next simpler one.
+int launch_schedule(int mode, const layout& P, int64_t work_bytes) {
+    const bool automatic = mode == 0;
+    if (automatic) mode = automatic_mode(int(P.C));
+    if (mode == 5 && (P.Cp / kT < 4 || (automatic && work_bytes < P.flow_total))) mode = 3;
+    if ((mode == 6 || mode == 8) && (P.Cp / kT < 2 || (automatic && work_bytes < P.flow_total))) mode = 1;
+    return mode;
+}
+
+// The wide micro-tile is for 16-bit lanes: what the schedules that differ in it alone are in 32-bit ones.
+int schedule_in_lanes(int mode, int lane_bits) {
+    if (lane_bits != 32) return mode;
+    return mode == 3 || mode == 4 || mode == 7 ? 1 : mode == 8 ? 6 : mode;
+}
+
+// Whether the automatic schedule tries the resident closure first.
+bool resident_first(int C, int lane_bits, int64_t work_bytes) {
+    return g_closure_mode.load() == 0 && C <= resident::max_candidates(lane_bits) &&
+           work_bytes >= resident::workspace_bytes(C, lane_bits);
+}
+
+// What the calling thread's last closure call queued: 1 to 8, SE_CLOSURE_RESIDENT, or 0 where it failed before.
+thread_local int g_last_schedule = 0;
+
 template <int LB> se_status_t set_smem_limits() {
     const int bytes = int(batch::pcfg<LB>::SMEM);
     auto raise = [bytes](const void* fn, const char* what) { return raise_smem_limit(fn, bytes, what); };
@@ -1275,6 +1300,7 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
                         int lane_bits, uint32_t value_offset, int tile, void* d_work, int64_t work_bytes,
                         void* stream_, double* phase_ms, int mode_override, bool sync) {
     clear_error();
+    g_last_schedule = 0;
     SE_REQUIRE(C >= 1, SE_ERR_INVALID, "Number of candidates must be positive");
     SE_REQUIRE(C <= (1 << 20), SE_ERR_INVALID, "Number of candidates too large (%d)", C);
     SE_REQUIRE(d_pref && d_out, SE_ERR_INVALID, "null matrix pointer");
@@ -1305,6 +1331,7 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
         if (se_status_t st = resident::run(d_pref, ld_pref, C, d_out, ld_out, bits, base, lane_bits == 0, work,
                                            work_bytes, s, &ran))
             return st;
+        if (ran) g_last_schedule = SE_CLOSURE_RESIDENT;
         if (ran && lane_bits == 0) {
             uint32_t words[resident::kWide + 1] = {};
             SE_CUDA_TRY(cudaMemcpyAsync(words, work, sizeof(words), cudaMemcpyDeviceToHost, s));
@@ -1350,9 +1377,7 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
     } else {
         if (se_status_t st = launch_init<32>(d_pref, ld_pref, C, P, work, 0, s)) return st;
     }
-    if (automatic) mode = automatic_mode(C);
-    if (mode == 5 && (P.Cp / kT < 4 || (automatic && work_bytes < P.flow_total))) mode = 3;
-    if ((mode == 6 || mode == 8) && (P.Cp / kT < 2 || (automatic && work_bytes < P.flow_total))) mode = 1;
+    mode = launch_schedule(mode, P, work_bytes);
     const bool flow = mode == 2 && P.Cp > kT;
     SE_REQUIRE((mode != 2 && mode != 5 && mode != 6 && mode != 8) || work_bytes >= P.flow_total, SE_ERR_WORKSPACE,
                "the dataflow, two-stream and one-launch-per-round closures need a workspace of %lld bytes",
@@ -1361,6 +1386,7 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
                           : (lb == 16 ? run_rounds<16>(work, P, s, phase_ms, mode, work_bytes >= P.flow_total)
                                       : run_rounds<32>(work, P, s, phase_ms, mode, work_bytes >= P.flow_total));
     if (st) return st;
+    g_last_schedule = schedule_in_lanes(mode, lb);
     st = lb == 16 ? launch_finalize<16>(P, work, C, d_out, ld_out, base, s)
                   : launch_finalize<32>(P, work, C, d_out, ld_out, 0, s);
     if (st) return st;
@@ -1381,6 +1407,22 @@ se_status_t report_flags(const uint32_t* flags) {
     SE_REQUIRE(flags[0] == 0, SE_ERR_DEVICE, "closure kernel reported device error %u (TMA wait timed out)",
                flags[0]);
     return SE_OK;
+}
+}  // namespace closure
+}  // namespace se
+
+namespace se {
+namespace closure {
+// Kernels of one closure through the launches: init, pivot of round 0, R x (panels, remainder),
+// finalize; mode 4 adds a pivot launch per later round (in 16-bit lanes), mode 5 a second remainder
+// launch per round but the last; 6 and 8 run init, pivot, panels 0, R - 1 rounds, last, finalize.
+int launches_of_schedule(int C) {
+    if (C < 1) return 0;
+    const int R = int(round_up(C, kT) / kT);
+    int mode = g_closure_mode.load();
+    if (mode == 0) mode = automatic_mode(C);
+    if ((mode == 6 || mode == 8) && R >= 2) return 3 + R + 1;
+    return R == 1 ? 3 : 3 + 2 * R + (mode == 4 || (mode == 5 && R >= 4) ? R - 1 : 0);
 }
 }  // namespace closure
 }  // namespace se
@@ -1417,7 +1459,7 @@ extern "C" se_status_t se_closure_profiled(const uint32_t* d_pref, int64_t ld_pr
         return closure_run(d_pref, ld_pref, C, d_out, ld_out, lane_bits, 0, tile, d_work, work_bytes, stream, phase_ms,
                            -1, true);
     });
-    if (launches) *launches = se_closure_launch_count(C);
+    if (launches) *launches = launches_of_schedule(C);
     return st;
 }
 
@@ -1450,15 +1492,14 @@ extern "C" se_status_t se_closure_set_mode(int mode) {
 extern "C" int se_closure_schedule(int C, int lane_bits, int64_t work_bytes) {
     if (C < 1) return -1;
     const layout P = plan(C, lane_bits == 32 ? 32 : 16);
-    int mode = g_closure_mode.load();
-    const bool automatic = mode == 0;
-    if (automatic) mode = automatic_mode(C);
-    if (mode == 5 && (P.Cp / kT < 4 || (automatic && work_bytes < P.flow_total))) mode = 3;
-    if ((mode == 6 || mode == 8) && (P.Cp / kT < 2 || (automatic && work_bytes < P.flow_total))) mode = 1;
-    if (lane_bits == 32 && (mode == 3 || mode == 4 || mode == 7)) mode = 1;
-    if (lane_bits == 32 && mode == 8) mode = 6;
-    return mode;
+    return schedule_in_lanes(launch_schedule(g_closure_mode.load(), P, work_bytes), lane_bits);
 }
+
+extern "C" int se_closure_resident(int C, int lane_bits, int64_t work_bytes) {
+    return C >= 1 && resident_first(C, lane_bits == 32 ? 32 : 16, work_bytes) ? 1 : 0;
+}
+
+extern "C" int se_closure_last_schedule(void) { return g_last_schedule; }
 
 extern "C" se_status_t se_closure_set_variant_table(const int* max_c, const int* modes, int n) {
     return host_guard([&]() -> se_status_t {
@@ -1479,12 +1520,6 @@ extern "C" se_status_t se_closure_set_variant_table(const int* max_c, const int*
 }
 
 extern "C" int se_closure_launch_count(int C) {
-    if (C < 1) return 0;
-    const int R = int(round_up(C, kT) / kT);
-    int mode = g_closure_mode.load();
-    if (mode == 0) mode = automatic_mode(C);
-    // init, pivot of round 0, R x (panels, remainder), finalize; mode 4 adds a pivot launch
-    // per later round (in 16-bit lanes), mode 5 a second remainder launch per round but the last.
-    if ((mode == 6 || mode == 8) && R >= 2) return 3 + R + 1;  // init, pivot, panels 0, R - 1 rounds, last, finalize
-    return R == 1 ? 3 : 3 + 2 * R + (mode == 4 || (mode == 5 && R >= 4) ? R - 1 : 0);
+    if (C >= 1 && resident_first(C, 16, se_closure_workspace_bytes_flow(C, 16, 0))) return 1;
+    return launches_of_schedule(C);
 }
