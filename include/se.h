@@ -125,7 +125,11 @@ SE_API se_status_t se_closure_profiled(const uint32_t* d_pref, int64_t ld_pref, 
  * also holds the panel buffers of the resident closure (up to 16 MiB more than the plain size):
  * one launch that keeps the whole matrix in the SMs' registers, which the automatic schedule
  * then runs in place of the schedules below (identical results), except into a capturing
- * stream. */
+ * stream. That launch needs all its CTAs on the GPU at once. Where kernels of other streams keep
+ * the SMs that it needs for longer than 1 ms, it gives way before it writes anything, and the
+ * schedules below run instead, as they did in the room that is left (se_closure_enqueue: the
+ * dataflow form, queued behind it; it takes the resident closure for 1 to 64 candidates and from
+ * 129 on). */
 SE_API int64_t se_closure_workspace_bytes_flow(int C, int lane_bits, int tile);
 
 /* Task t (< R^3) of the dataflow closure's fixed order for R = ceil(C / 128) pivot blocks:
@@ -183,6 +187,11 @@ SE_API int se_closure_resident(int C, int lane_bits, int64_t work_bytes);
  * it failed before it queued one or there was no call. */
 #define SE_CLOSURE_RESIDENT 9
 SE_API int se_closure_last_schedule(void);
+
+/* How long, in the calling thread's later closure calls, the CTAs of a resident closure wait for all
+ * of them to be on the GPU before it gives way (1000000 at first). 0: it always gives way,
+ * except as a single CTA (C <= 64). Results are the same either way. */
+SE_API void se_closure_set_start_limit(uint64_t limit_ns);
 
 /* Number of kernels one se_closure call launches for C candidates in 16-bit lanes, with
  * se_closure_workspace_bytes_flow() of workspace, under the current schedule (automatic lanes add

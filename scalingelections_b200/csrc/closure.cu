@@ -410,11 +410,19 @@ __host__ __device__ FlowTask flow_decode(uint32_t t_in, int R) {
     return T;
 }
 
+// Kernels that stand behind a resident launch take its check-in word as their gate: they run where
+// it gave way (closure_resident.cu) and return at once where it did not. No gate: they run. Gated ones
+// are programmatic dependent launches, so that the next one is ready when one returns.
+__device__ __forceinline__ bool open_gate(const uint32_t* gate) { return !gate || (*gate & resident::kGaveWay); }
+
 template <int LB>
 __global__ void __launch_bounds__(cfg<LB>::THREADS, 1)
     flow_kernel(const __grid_constant__ batch::Elec E0, const __grid_constant__ batch::Elec E1,
-                uint32_t* __restrict__ state, uint32_t* __restrict__ err) {
+                uint32_t* __restrict__ state, uint32_t* __restrict__ err, const uint32_t* __restrict__ gate) {
     using CF = cfg<LB>;
+    pdl_trigger();
+    pdl_wait();
+    if (!open_gate(gate)) return;
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(16) uint32_t rowbuf[kPivotBufs][CF::TW];
     __shared__ __align__(16) uint32_t colbuf[kPivotBufs][kT];
@@ -540,7 +548,13 @@ __global__ void __launch_bounds__(tile_threads<LB, NQ>(), 1)
 template <int LB>
 __global__ void __launch_bounds__(256)
     init_kernel(const uint32_t* __restrict__ d, int64_t ld, int C, int Cp, void* __restrict__ Sv, uint32_t base,
-                uint32_t* __restrict__ flags) {
+                uint32_t* __restrict__ flags, const uint32_t* __restrict__ gate, uint32_t* __restrict__ clear,
+                int clear_words) {
+    pdl_trigger();
+    pdl_wait();
+    if (!open_gate(gate)) return;
+    if (blockIdx.x == 0 && blockIdx.y == 0)  // the words that the next launch counts in
+        for (int w = threadIdx.y * 32 + threadIdx.x; w < clear_words; w += 256) clear[w] = 0u;
     __shared__ uint32_t t[32][33];
     const int bx = blockIdx.x * 32, by = blockIdx.y * 32;  // this block writes S[by.., bx..]
     // Stage d[bx + y][by + x] (the transposed block) so t[x][y] = d[bx + y][by + x].
@@ -635,8 +649,9 @@ __global__ void __launch_bounds__(256, kRangeCtasPerSm)
 template <int LB>
 __global__ void __launch_bounds__(256)
     finalize_kernel(const void* __restrict__ Sv, int Cp, int C, uint32_t* __restrict__ out, int64_t ld_out,
-                    uint32_t base) {
+                    uint32_t base, const uint32_t* __restrict__ gate) {
     pdl_wait();  // the closure's last launch is complete and visible
+    if (!open_gate(gate)) return;
     const bool vec = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     for (int i = blockIdx.y; i < C; i += gridDim.y)
         for (int j = 4 * (blockIdx.x * blockDim.x + threadIdx.x); j < C; j += 4 * gridDim.x * blockDim.x) {
@@ -832,11 +847,11 @@ template <int LB> se_status_t set_smem_limits() {
 // that the previous grid's last, partial wave leaves free and start its first tiles the moment
 // that grid completes, without the launch gap.
 template <typename... Params, typename... Args>
-void launch_pdl(bool pdl, void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+void launch_pdl(bool pdl, void (*kernel)(Params...), dim3 grid, dim3 threads, size_t smem, cudaStream_t s,
                 Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(unsigned(threads));
+    cfg.blockDim = threads;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1166,9 +1181,12 @@ se_status_t run_rounds(uint8_t* work, const layout& P, cudaStream_t stream, doub
     return SE_OK;
 }
 
-// The dataflow closure on an initialised working matrix (pivot of round 0 included).
+// The dataflow closure on an initialised working matrix (pivot of round 0 included). Behind a gate the
+// init launch clears its state.
+int flow_state_words(int R) { return 4 + R * R + 2 * R; }
 template <int LB>
-se_status_t run_flow(uint8_t* work, const layout& P, cudaStream_t stream, double* phase_ms) {
+se_status_t run_flow(uint8_t* work, const layout& P, cudaStream_t stream, double* phase_ms,
+                     const uint32_t* gate = nullptr) {
     using CF = cfg<LB>;
     if (se_status_t st = set_smem_limits<LB>(); st != SE_OK) return st;
     uint32_t* S = reinterpret_cast<uint32_t*>(work + P.s_off);
@@ -1193,7 +1211,7 @@ se_status_t run_flow(uint8_t* work, const layout& P, cudaStream_t stream, double
         E[b].lanes = LB;
     }
     uint32_t* state = reinterpret_cast<uint32_t*>(work + P.state_off);
-    SE_CUDA_TRY(cudaMemsetAsync(state, 0, size_t(4 + R * R + 2 * R) * 4, stream));
+    if (!gate) SE_CUDA_TRY(cudaMemsetAsync(state, 0, size_t(flow_state_words(R)) * 4, stream));
     int device = 0, sms = 0, occ = 0;
     SE_CUDA_TRY(cudaGetDevice(&device));
     SE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -1208,7 +1226,8 @@ se_status_t run_flow(uint8_t* work, const layout& P, cudaStream_t stream, double
         cudaEventCreate(&e1);
         cudaEventRecord(e0, stream);
     }
-    flow_kernel<LB><<<grid, CF::THREADS, batch::pcfg<LB>::SMEM, stream>>>(E[0], E[1], state, err);
+    launch_pdl(gate != nullptr, flow_kernel<LB>, unsigned(grid), CF::THREADS, batch::pcfg<LB>::SMEM, stream, E[0],
+               E[1], state, err, gate);
     SE_CHECK_LAUNCH();
     if (phase_ms) {
         cudaEventRecord(e1, stream);
@@ -1226,21 +1245,23 @@ se_status_t run_flow(uint8_t* work, const layout& P, cudaStream_t stream, double
 
 template <int LB>
 se_status_t launch_init(const uint32_t* d, int64_t ld, int C, const layout& P, uint8_t* work, uint32_t base,
-                        cudaStream_t s) {
+                        cudaStream_t s, const uint32_t* gate = nullptr) {
     const int nb = int(P.Cp / 32);
-    init_kernel<LB><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(d, ld, C, int(P.Cp), work + P.s_off, base,
-                                                       reinterpret_cast<uint32_t*>(work + P.flags_off));
+    launch_pdl(gate != nullptr, init_kernel<LB>, dim3(nb, nb), dim3(32, 8), 0, s, d, ld, C, int(P.Cp),
+               static_cast<void*>(work + P.s_off), base, reinterpret_cast<uint32_t*>(work + P.flags_off), gate,
+               gate ? reinterpret_cast<uint32_t*>(work + P.state_off) : nullptr,
+               gate ? flow_state_words(int(P.Cp / kT)) : 0);
     SE_CHECK_LAUNCH();
     return SE_OK;
 }
 
 template <int LB>
 se_status_t launch_finalize(const layout& P, uint8_t* work, int C, uint32_t* out, int64_t ld_out, uint32_t base,
-                            cudaStream_t s) {
+                            cudaStream_t s, const uint32_t* gate = nullptr) {
     const int gx = int((C + 1023) / 1024);
-    const int gy = C < 65535 ? C : 65535;
+    const int gy = gate ? (C + 7) / 8 : C < 65535 ? C : 65535;  // a gated launch's usual work is to return
     launch_pdl(true, finalize_kernel<LB>, dim3(unsigned(gx), unsigned(gy)), 256, 0, s,
-               static_cast<const void*>(work + P.s_off), int(P.Cp), C, out, ld_out, base);
+               static_cast<const void*>(work + P.s_off), int(P.Cp), C, out, ld_out, base, gate);
     SE_CHECK_LAUNCH();
     return SE_OK;
 }
@@ -1251,9 +1272,9 @@ se_status_t launch_defeat_init(const uint32_t* d, int64_t ld, int C, int Cp, voi
                                uint32_t* flags, cudaStream_t s) {
     const int nb = Cp / 32;
     if (lane_bits == 16)
-        init_kernel<16><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(d, ld, C, Cp, S, base, flags);
+        init_kernel<16><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(d, ld, C, Cp, S, base, flags, nullptr, nullptr, 0);
     else
-        init_kernel<32><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(d, ld, C, Cp, S, 0, flags);
+        init_kernel<32><<<dim3(nb, nb), dim3(32, 8), 0, s>>>(d, ld, C, Cp, S, 0, flags, nullptr, nullptr, 0);
     SE_CHECK_LAUNCH();
     return SE_OK;
 }
@@ -1291,6 +1312,18 @@ se_status_t prepare_launches(int lane_bits) {
     return SE_OK;
 }
 
+// The launches behind a resident launch that nobody waits for: the dataflow form, which is three (8 us for
+// all three where they return at once: 91 -> 99 us a queued closure at C = 517, 447 -> 455 at 1500).
+template <int LB>
+se_status_t queue_gated(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, uint32_t base,
+                        uint8_t* work, cudaStream_t s) {
+    const layout P = plan(C, LB);
+    const uint32_t* gate = reinterpret_cast<const uint32_t*>(work) + resident::kArrived;
+    if (se_status_t st = launch_init<LB>(d, ld, C, P, work, base, s, gate)) return st;
+    if (se_status_t st = run_flow<LB>(work, P, s, nullptr, gate)) return st;
+    return launch_finalize<LB>(P, work, C, out, ld_out, base, s, gate);
+}
+
 // The closure behind every entry point. mode: 0/1 round by round, 2 dataflow, -1 the
 // process-wide choice (se_closure_set_mode). sync: read the flags back and report overflow or
 // a device error (else the call is stream-ordered and se_closure_check reports them later).
@@ -1322,28 +1355,32 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
     uint32_t base = value_offset;
     int mode = mode_override >= 0 ? mode_override : g_closure_mode.load();
     const bool automatic = mode == 0;
-    if (automatic && phase_ms == nullptr) {
-        // Matrices that fit the SMs' register files close in one launch (closure_resident.cu): 1.4 to
-        // 2.1 times faster than the launches below at every size that it takes (its shapes' table).
+    // Matrices that fit the SMs' register files close in one launch (closure_resident.cu): 1.4 to
+    // 2.1 times faster than the launches below at every size that it takes (its shapes' table).
+    // That launch may give way where other kernels hold the SMs that it needs. A call that waits
+    // then runs the launches; one that only queues has queued gated launches behind it, so it needs
+    // room for them, and a second pivot block for that form to apply.
+    if (automatic && phase_ms == nullptr &&
+        (sync || resident::single_cta(C) || (C > kT && work_bytes >= plan(C, lb).flow_total))) {
         if (se_status_t st = prepare_launches(lane_bits)) return st;
-        bool ran = false;
-        int bits = lb;
-        if (se_status_t st = resident::run(d_pref, ld_pref, C, d_out, ld_out, bits, base, lane_bits == 0, work,
-                                           work_bytes, s, &ran))
-            return st;
-        if (ran) g_last_schedule = SE_CLOSURE_RESIDENT;
-        if (ran && lane_bits == 0) {
-            uint32_t words[resident::kWide + 1] = {};
+        for (;;) {
+            bool ran = false;
+            if (se_status_t st = resident::run(d_pref, ld_pref, C, d_out, ld_out, lb, base, lane_bits == 0, work,
+                                               work_bytes, s, &ran))
+                return st;
+            if (!ran) break;
+            g_last_schedule = SE_CLOSURE_RESIDENT;
+            if (!sync)
+                return resident::single_cta(C) ? SE_OK
+                       : lb == 16 ? queue_gated<16>(d_pref, ld_pref, C, d_out, ld_out, base, work, s)
+                                  : queue_gated<32>(d_pref, ld_pref, C, d_out, ld_out, 0, work, s);
+            uint32_t words[resident::kArrived + 1] = {};
             SE_CUDA_TRY(cudaMemcpyAsync(words, work, sizeof(words), cudaMemcpyDeviceToHost, s));
             SE_CUDA_TRY(cudaStreamSynchronize(s));
+            if (words[resident::kArrived] & resident::kGaveWay) break;
             if (words[resident::kWide] == 0u) return report_flags(words);
-            bits = lane_bits = 32;  // no 16-bit window holds the kept counts
-            if (se_status_t st = resident::run(d_pref, ld_pref, C, d_out, ld_out, bits, 0, false, work, work_bytes, s,
-                                               &ran))
-                return st;
-            lb = 32;
+            lb = lane_bits = 32;  // no 16-bit window holds the kept counts
         }
-        if (ran) return sync ? check_flags(work, s) : SE_OK;
     }
     SE_CUDA_TRY(cudaMemsetAsync(work, 0, 256, s));
     if (lane_bits == 0) {
@@ -1488,6 +1525,8 @@ extern "C" se_status_t se_closure_set_mode(int mode) {
     g_closure_mode.store(mode);
     return SE_OK;
 }
+
+extern "C" void se_closure_set_start_limit(uint64_t limit_ns) { resident::set_start_limit(limit_ns); }
 
 extern "C" int se_closure_schedule(int C, int lane_bits, int64_t work_bytes) {
     if (C < 1) return -1;

@@ -38,6 +38,13 @@
 // product reads them); two publishers, for the row and the columns, raise the flags of the CTA's
 // own blocks, so that no compute warp waits for a fence.
 //
+// All CTAs of the launch have to be on the GPU at once, and kernels of other streams may hold SMs for
+// as long as they like. So the CTAs check in before the first round (all_here): if they are not all
+// there within a limit, the launch gives way, that is, every CTA leaves before anything is
+// written but flags, and the closure runs as launches, which take the room there is: started by
+// the host where the call waits, or by kernels queued behind this one that otherwise return at
+// once (closure.cu). A checked-in launch has its SMs until it ends.
+//
 // Every wait is bounded. A wait that runs out records an error and makes its thread stop waiting,
 // not stop: control flow stays uniform, every CTA reaches the end, and the host reports the error.
 #include <cuda_runtime.h>
@@ -64,7 +71,7 @@ constexpr int kThreads = kNT + 96;  // and the helper warps: the producer and tw
 
 // Words of the flags area at the start of the workspace. 0 and 1 are the closure's common words
 // (device error, 16-bit overflow).
-constexpr int kWordErr = 0, kWordOverflow = 1, kWordLo = 2, kWordHi = 3, kWordWide = kWide, kWordArrived = 5;
+constexpr int kWordErr = 0, kWordOverflow = 1, kWordLo = 2, kWordHi = 3, kWordWide = kWide, kWordArrived = kArrived;
 
 // Thread geometry: the compute threads share every 64 x 64 block evenly, 4 x 4 cells each: thread
 // (tr, tc) owns rows 4 tr .. and cells 4 tc .. of each of the CTA's blocks. A warp is 4 x 8 threads:
@@ -157,7 +164,31 @@ struct Params {
     int C, NB, NR, tiles_j;
     uint32_t base;     // 16-bit lanes store a kept value v as v - base (see init_kernel in closure.cu)
     int automatic;     // choose the 16-bit window here; give up (kWordWide) when none holds
+    uint64_t start_ns; // the check-in's limit
 };
+
+// One thread of each CTA checks in and waits for the others. All of them see the same outcome: a wait
+// that runs out can mark the word only as long as a CTA is missing from its count, and a marked
+// count never serves as a full one.
+__device__ __forceinline__ bool all_here(uint32_t* arrived, uint32_t n, uint64_t limit_ns) {
+    if (limit_ns == 0u && n > 1u) {  // no wait at all, for every CTA alike
+        atomicOr(arrived, kGaveWay);
+        return false;
+    }
+    __threadfence();
+    uint32_t seen = atomicAdd(arrived, 1u) + 1u;
+    const uint64_t t0 = global_ns();
+    for (uint32_t it = 0; seen != n && !(seen & kGaveWay); ++it) {
+        if ((it & 63u) == 0u && global_ns() - t0 >= limit_ns) {
+            const uint32_t old = atomicCAS(arrived, seen, seen | kGaveWay);
+            seen = old == seen ? seen | kGaveWay : old;
+        } else {
+            seen = ld_acquire_gpu(arrived);
+        }
+    }
+    __threadfence();
+    return seen == n;
+}
 
 // c[r][q] = max(c[r][q], max_k min(A[k][row], B[k][word])) over kn pivots (a multiple of 4). a and
 // b point at the thread's row and word; PA and PB are the operands' pitches.
@@ -437,10 +468,10 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
 
     // ---- Helper warps. ----
     if (warp >= kNT / 32) {
-        if (P.automatic) {
-            __syncthreads();  // the window is agreed on
-            if (!s_go) return;
-        }
+        if (!P.automatic && warp == kNT / 32 && lane == 0 && !all_here(P.words + kWordArrived, gridDim.x, P.start_ns))
+            s_go = 0u;
+        __syncthreads();  // every CTA is here and, with automatic lanes, the window is agreed on
+        if (!s_go) return;
         const int role = warp - kNT / 32;
         if (role == 0) {
             // Producer: lane x watches slot x; lane 0 alone fills them (a bulk copy's operands are
@@ -576,30 +607,25 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
                     atomicMax(P.words + kWordLo, ~s_lo);  // the area starts at zero
                     atomicMax(P.words + kWordHi, s_hi);
                 }
-                __threadfence();
-                atomicAdd(P.words + kWordArrived, 1u);
-                const uint64_t t0 = global_ns();
-                bool ok = true;
-                for (uint32_t it = 1; ok && ld_acquire_gpu(P.words + kWordArrived) < gridDim.x; ++it)
-                    if ((it & 255u) == 0u && global_ns() - t0 > kWaitNs) ok = false;
-                const uint32_t ghi = ld_acquire_gpu(P.words + kWordHi), glo = ~ld_acquire_gpu(P.words + kWordLo);
-                if (!ok) {
-                    raise_device_error(P.words + kWordErr, kErrTmaTimeout);
+                if (!all_here(P.words + kWordArrived, gridDim.x, P.start_ns)) {
                     s_go = 0u;
-                } else if (ghi > 0xFFFFu) {
-                    if (ghi - glo < 0xFFFFu) s_base = glo - 1u;
-                    else s_go = 0u;
-                    if (!s_go && blockIdx.x == 0) P.words[kWordWide] = 1u;
+                } else {
+                    const uint32_t ghi = ld_acquire_gpu(P.words + kWordHi), glo = ~ld_acquire_gpu(P.words + kWordLo);
+                    if (ghi > 0xFFFFu) {
+                        if (ghi - glo < 0xFFFFu) s_base = glo - 1u;
+                        else s_go = 0u;
+                        if (!s_go && blockIdx.x == 0) P.words[kWordWide] = 1u;
+                    }
                 }
-            }
-            __syncthreads();  // with the helper warps
-            if (!s_go) return;
-            if (s_base != base) {
-                base = s_base;
-                load();
             }
         } else if (LB == 16 && over) {
             atomicOr(P.words + kWordOverflow, 1u);
+        }
+        __syncthreads();  // with the helper warps
+        if (!s_go) return;
+        if (s_base != base) {
+            base = s_base;
+            load();
         }
     }
 
@@ -988,6 +1014,13 @@ se_status_t leave(Order& o, cudaStream_t s) {
     return SE_OK;
 }
 
+// The check-in's limit, of the calling thread's launches. Once the CTAs that there is room for spin, the
+// time is lost to everyone, so it is about what the launches take longer than the resident form
+// (0.1 to 0.3 ms); CTAs that find room come within some 10 us, so this limit is for other kernels to end.
+constexpr uint64_t kStartNs = 1000000ull;
+thread_local uint64_t g_start_ns = kStartNs;
+void set_start_limit(uint64_t ns) { g_start_ns = ns; }
+
 se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, int lane_bits, uint32_t base,
                 bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, bool* ran) {
     *ran = false;
@@ -1022,6 +1055,7 @@ se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_
     P.tiles_j = int((L.NB + sh->cb - 1) / sh->cb);
     P.base = base;
     P.automatic = automatic ? 1 : 0;
+    P.start_ns = g_start_ns;
     SE_CUDA_TRY(cudaMemsetAsync(work, 0, size_t(L.zero_bytes), s));
 
     cudaLaunchConfig_t cfg = {};

@@ -21,11 +21,18 @@ int64_t workspace_bytes(int C, int lane_bits);
 // Queues the whole closure on s and sets *ran, or leaves *ran false where the resident form does
 // not apply (size, workspace, device, a capturing stream). The first two words of the workspace
 // are the closure's flags, as in closure.cu. automatic: 16-bit lanes with the window chosen on
-// the device; where none holds, word kWide is set and nothing is written to out.
+// the device; where none holds, word kWide is set and nothing is written to out. Where the CTAs were
+// not all on the GPU in time, word kArrived has bit kGaveWay and nothing is written to out either.
 se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, int lane_bits, uint32_t base,
                 bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, bool* ran);
 
-constexpr int kWide = 4;
+constexpr int kWide = 4, kArrived = 5;
+constexpr uint32_t kGaveWay = 0x80000000u;
+
+// Whether a launch for C candidates is a single CTA, which cannot give way.
+constexpr bool single_cta(int C) { return C <= kB; }
+
+void set_start_limit(uint64_t ns);
 
 }  // namespace resident
 }  // namespace se
