@@ -193,6 +193,11 @@ SE_API int se_closure_last_schedule(void);
  * except as a single CTA (C <= 64). Results are the same either way. */
 SE_API void se_closure_set_start_limit(uint64_t limit_ns);
 
+/* Limit, in the calling thread's later closure calls, of one wait between the CTAs of a resident
+ * closure that has not given way (2 s at first, 10 s at most; 0: a wait takes one look). A wait that
+ * runs out, which only a broken launch does, ends the call with SE_ERR_DEVICE; the GPU stays usable. */
+SE_API void se_closure_set_wait_limit(uint64_t limit_ns);
+
 /* Number of kernels one se_closure call launches for C candidates in 16-bit lanes, with
  * se_closure_workspace_bytes_flow() of workspace, under the current schedule (automatic lanes add
  * at most one more): 1 where the resident closure runs. */

@@ -1528,6 +1528,8 @@ extern "C" se_status_t se_closure_set_mode(int mode) {
 
 extern "C" void se_closure_set_start_limit(uint64_t limit_ns) { resident::set_start_limit(limit_ns); }
 
+extern "C" void se_closure_set_wait_limit(uint64_t limit_ns) { resident::set_wait_limit(limit_ns); }
+
 extern "C" int se_closure_schedule(int C, int lane_bits, int64_t work_bytes) {
     if (C < 1) return -1;
     const layout P = plan(C, lane_bits == 32 ? 32 : 16);

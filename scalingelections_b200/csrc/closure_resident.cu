@@ -46,7 +46,10 @@
 // once (closure.cu). A checked-in launch has its SMs until it ends.
 //
 // Every wait is bounded. A wait that runs out records an error and makes its thread stop waiting,
-// not stop: control flow stays uniform, every CTA reaches the end, and the host reports the error.
+// not stop: control flow stays uniform, every CTA reaches the end, and the host reports the error. A
+// thread that has given up arrives on no barrier of the slots any more, so nobody who still waits is
+// told that a slot is full or free when it is not, and no barrier gets more arrivals than it counts. The
+// producer that gives up starts no more copies and waits for those that it started.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -64,7 +67,7 @@ using closure::kErrTmaTimeout;
 using closure::ld4;
 using closure::st4;
 
-constexpr uint64_t kWaitNs = 2000000000ull;  // one wait
+constexpr uint64_t kWaitNs = 2000000000ull;  // one wait, unless the caller sets another limit
 constexpr int kP = 32;               // pivots per round
 constexpr int kNT = 256;             // compute threads
 constexpr int kThreads = kNT + 96;  // and the helper warps: the producer and two publishers
@@ -149,6 +152,7 @@ __device__ __forceinline__ void sync_pair(int pair) { sync_threads<64>(2 + pair)
 __device__ __forceinline__ void sync_rows(int h) { sync_threads<128>(6 + h); }
 __device__ __forceinline__ void sync_cols(int h) { sync_threads<128>(8 + h); }
 constexpr int kBarD = 10, kBarSides = 11;  // the diagonal block's D is there; its other two pieces are
+constexpr int kBarEnd = 12;                // the compute warps are done with the slots
 
 struct Params {
     const uint32_t* d;
@@ -165,6 +169,8 @@ struct Params {
     uint32_t base;     // 16-bit lanes store a kept value v as v - base (see init_kernel in closure.cu)
     int automatic;     // choose the 16-bit window here; give up (kWordWide) when none holds
     uint64_t start_ns; // the check-in's limit
+    uint64_t wait_ns;  // the limit of any wait after it; 0: one look
+    uint32_t polls;    // and that of a wait on an mbarrier
 };
 
 // One thread of each CTA checks in and waits for the others. All of them see the same outcome: a wait
@@ -431,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
     constexpr bool kEarly = CB == 1;  // diagonal() runs two rounds ahead
     extern __shared__ __align__(1024) uint32_t smem[];
     __shared__ uint64_t full[kStages][1 + CB], empty[kStages];  // slot 0 is A, slot 1 + y is B[y]
-    __shared__ uint32_t s_lo, s_hi, s_base, s_go;
+    __shared__ uint32_t s_lo, s_hi, s_base, s_go, s_dead;
     __shared__ uint32_t prog_row[kNT / 32], prog_col[kNT / 32];  // panel blocks stored, per warp
     const int I = blockIdx.x / P.tiles_j, J = blockIdx.x % P.tiles_j;
     const int NB = P.NB, NR = P.NR;
@@ -445,6 +451,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
         s_lo = 0xFFFFFFFFu;
         s_hi = 0u;
         s_go = 1u;
+        s_dead = 0u;
         s_base = P.base;
     }
     if (tid < kNT / 32) prog_row[tid] = prog_col[tid] = 0u;
@@ -476,18 +483,18 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
         if (role == 0) {
             // Producer: lane x watches slot x; lane 0 alone fills them (a bulk copy's operands are
             // warp-uniform, so one lane at a time may issue it).
-            bool dead = false;              // uniform, as all below
-            uint64_t copied = 0;            // 16 bits per stage: slots whose newest phase is a copy
+            bool dead = false;              // a wait ran out (uniform, as all below)
+            uint64_t copied = 0;            // 16 bits per stage: slots copied into, and the last copy's phase
             const uint32_t empty_blocks = ((1u << (1 + CB)) - 1u) & ~((1u << (1 + nc)) - 1u);
-            for (int k = 0; k < NR; ++k) {
+            for (int k = 0; k < NR && !dead; ++k) {
                 const int s = k % kStages;
                 // The compute warps fill the slots of the CTA's own panel blocks.
                 uint32_t pending = (in_cols(k) ? 0u : 1u) | (in_rows(k) ? 0u : ((1u << nc) - 1u) << 1);
-                if ((pending | empty_blocks) && k >= kStages && !dead)
-                    dead = __any_sync(0xFFFFFFFFu, !mbar_wait_bounded(&empty[s], uint32_t(k / kStages - 1) & 1u, 1u << 26, kWaitNs));
+                if ((pending | empty_blocks) && k >= kStages)
+                    dead = __any_sync(0xFFFFFFFFu,
+                                      !mbar_wait_bounded(&empty[s], uint32_t(k / kStages - 1) & 1u, P.polls, P.wait_ns));
+                if (dead) break;
                 const uint32_t* flag = lane == 0 ? P.flag_a + k * NB + I : P.flag_b + k * NB + J * CB + lane - 1;
-                uint32_t fill = empty_blocks | (dead ? pending : 0u);  // phases to complete without a copy
-                if (dead) pending = 0u;
                 uint32_t got = 0u;
                 const uint64_t t0 = global_ns();
                 for (uint32_t it = 1; pending; ++it) {
@@ -508,28 +515,35 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
                         __syncwarp();
                         pending &= ~ready;
                         got |= ready;
-                    } else if ((it & 255u) == 0u && __any_sync(0xFFFFFFFFu, global_ns() - t0 > kWaitNs)) {
+                    } else if (P.wait_ns == 0u ||
+                               ((it & 255u) == 0u && __any_sync(0xFFFFFFFFu, global_ns() - t0 > P.wait_ns))) {
                         dead = true;
-                        fill |= pending;
-                        pending = 0u;
+                        break;
                     }
                 }
-                if (lane == 0) {
+                if (lane == 0 && !dead) {
                     for (int x = 0; x < 1 + CB; ++x)
-                        if ((fill >> x) & 1u) mbar_arrive(&full[s][x]);
-                    if (dead) raise_device_error(P.words + kWordErr, kErrTmaTimeout);
+                        if ((empty_blocks >> x) & 1u) mbar_arrive(&full[s][x]);  // a phase without a copy
                 }
                 __syncwarp();
-                copied = (copied & ~(0xFFFFull << (16 * s))) | (uint64_t(got) << (16 * s));
+                const uint32_t odd = (k / kStages) & 1 ? got : 0u;
+                copied = (copied & ~(uint64_t(got << 8) << (16 * s))) | (uint64_t(got | odd << 8) << (16 * s));
             }
-            // No copy outlives the CTA: the last phase of each stage has landed (bounded).
-            if (lane == 0) {
-                for (int k = NR > kStages ? NR - kStages : 0; k < NR; ++k) {
-                    const uint32_t got = uint32_t(copied >> (16 * (k % kStages))) & 0xFFFFu;
-                    for (int x = 0; x < 1 + CB; ++x)
-                        if ((got >> x) & 1u)
-                            mbar_wait_bounded(&full[k % kStages][x], uint32_t(k / kStages) & 1u, 1u << 26, kWaitNs);
-                }
+            if (dead && lane == 0) {
+                s_dead = 1u;
+                raise_device_error(P.words + kWordErr, kErrTmaTimeout);
+            }
+            // No copy outlives the CTA. The compute warps have waited for every slot of every round, unless one
+            // gave up: then the last copy into each slot is waited for here. (Where the compute warps filled
+            // that slot again it has landed, but its phase cannot be told from the next one, and the short
+            // limit runs out.)
+            sync_threads<kNT + 32>(kBarEnd);
+            if (lane == 0 && s_dead) {
+                for (int s = 0; s < kStages; ++s)
+                    for (int x = 0; x < 1 + CB; ++x) {
+                        const uint32_t c = uint32_t(copied >> (16 * s)) >> x;
+                        if (c & 1u) mbar_wait_bounded(&full[s][x], (c >> 8) & 1u, 1u << 26, kWaitNs / 1000);
+                    }
             }
         } else {
             // Publisher of the CTA's row blocks (role 1) or column blocks (role 2), in the order in
@@ -550,7 +564,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
                     const uint64_t since = global_ns();
                     bool ok = true;
                     for (uint32_t it = 1; !__all_sync(0xFFFFFFFFu, ld_acquire_smem(prog + w) >= key); ++it) {
-                        const bool late = (it & 255u) == 0u && global_ns() - since > 4 * kWaitNs;
+                        const bool late = P.wait_ns == 0u || ((it & 255u) == 0u && global_ns() - since > 4 * P.wait_ns);
                         if (__any_sync(0xFFFFFFFFu, late)) {
                             ok = false;
                             break;
@@ -631,11 +645,11 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
 
     bool dead = false;  // a wait of this thread ran out: it waits no more
     auto gave_up = [&]() {
-        raise_device_error(P.words + kWordErr, kErrTmaTimeout);
+        s_dead = 1u;
         dead = true;
     };
     auto wait_slot = [&](int k, int x) __attribute__((always_inline)) {
-        if (!dead && !mbar_wait_bounded(&full[k % kStages][x], uint32_t(k / kStages) & 1u, 1u << 26, 2 * kWaitNs))
+        if (!dead && !mbar_wait_bounded(&full[k % kStages][x], uint32_t(k / kStages) & 1u, P.polls, 2 * P.wait_ns))
             gave_up();
     };
     auto wait_b = [&](int k) __attribute__((always_inline)) {
@@ -645,7 +659,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
     // Every warp is done with the round that used k's stage before.
     auto wait_free = [&](int k) __attribute__((always_inline)) {
         if (!dead && k >= kStages &&
-            !mbar_wait_bounded(&empty[k % kStages], uint32_t(k / kStages - 1) & 1u, 1u << 26, 2 * kWaitNs))
+            !mbar_wait_bounded(&empty[k % kStages], uint32_t(k / kStages - 1) & 1u, P.polls, 2 * P.wait_ns))
             gave_up();
     };
     // A block's cells out of and back into the tile (y is uniform, the registers are static).
@@ -693,8 +707,9 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
             if (have && have2) break;
             if ((it & 255u) == 0u) {
                 const uint64_t now = global_ns();
-                if (it == 0) t0 = now;
-                else if (now - t0 > kWaitNs) gave_up();
+                if (P.wait_ns == 0u) gave_up();
+                else if (it == 0) t0 = now;
+                else if (now - t0 > P.wait_ns) gave_up();
             }
         }
     };
@@ -804,7 +819,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
         for (int y = 0; y < CB; ++y)
             if (y < nc) to_slot(c[y], y);
         sync_rows(h);
-        if (warp == (h ? 5 : 0) && lane == 0) {
+        if (warp == (h ? 5 : 0) && lane == 0 && !dead) {
             for (int y = 0; y < nc; ++y) mbar_arrive(&full[k % kStages][1 + y]);
         }
         for (int t = 0; t < nc; ++t) {
@@ -855,7 +870,7 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
             store_a<LB, kB>(w, slot);
         }
         sync_cols(h);
-        if (warp == h && lane == 0) mbar_arrive(&full[k % kStages][0]);
+        if (warp == h && lane == 0 && !dead) mbar_arrive(&full[k % kStages][0]);
         store_a<LB, kB>(w, block_a(k) + 4 * lc * kB + 4 * tr);
         __syncwarp();
         if (lane == 0) st_release_smem(&prog_col[warp], uint32_t(k) + 1u);
@@ -881,8 +896,11 @@ __global__ void __launch_bounds__(kThreads, OCC) resident_kernel(const __grid_co
         // This thread's slot writes come before the copies that follow.
         if (in_rows(k) || in_cols(k) || in_rows(k + 1) || in_cols(k + 1)) fence_proxy_async_all();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[k % kStages]);
+        if (lane == 0 && !dead) mbar_arrive(&empty[k % kStages]);
     }
+
+    if (dead) raise_device_error(P.words + kWordErr, kErrTmaTimeout);
+    arrive_threads<kNT + 32>(kBarEnd);
 
     // Output: widened, shifted back, zero on the diagonal (the reference's masks).
     const bool vec_out = P.ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(P.out) & 15) == 0;
@@ -1020,6 +1038,8 @@ se_status_t leave(Order& o, cudaStream_t s) {
 constexpr uint64_t kStartNs = 1000000ull;
 thread_local uint64_t g_start_ns = kStartNs;
 void set_start_limit(uint64_t ns) { g_start_ns = ns; }
+thread_local uint64_t g_wait_ns = kWaitNs;
+void set_wait_limit(uint64_t ns) { g_wait_ns = std::min(ns, 5 * kWaitNs); }
 
 se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, int lane_bits, uint32_t base,
                 bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, bool* ran) {
@@ -1056,6 +1076,8 @@ se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_
     P.base = base;
     P.automatic = automatic ? 1 : 0;
     P.start_ns = g_start_ns;
+    P.wait_ns = g_wait_ns;
+    P.polls = P.wait_ns ? 1u << 26 : 1u;
     SE_CUDA_TRY(cudaMemsetAsync(work, 0, size_t(L.zero_bytes), s));
 
     cudaLaunchConfig_t cfg = {};

@@ -33,6 +33,7 @@ constexpr uint32_t kGaveWay = 0x80000000u;
 constexpr bool single_cta(int C) { return C <= kB; }
 
 void set_start_limit(uint64_t ns);
+void set_wait_limit(uint64_t ns);
 
 }  // namespace resident
 }  // namespace se
