@@ -129,7 +129,9 @@ SE_API se_status_t se_closure_profiled(const uint32_t* d_pref, int64_t ld_pref, 
  * the SMs that it needs for longer than 1 ms, it gives way before it writes anything, and the
  * schedules below run instead, as they did in the room that is left (se_closure_enqueue: the
  * dataflow form, queued behind it; it takes the resident closure for 1 to 64 candidates and from
- * 129 on). */
+ * 129 on). Resident closures of different streams run at the same time where their CTAs (one
+ * per 64 x 64 cells, larger tiles from C = 1089 on) are no more than the SMs; one that does not fit
+ * beside those in flight takes the schedules below. No call waits for another stream. */
 SE_API int64_t se_closure_workspace_bytes_flow(int C, int lane_bits, int tile);
 
 /* Task t (< R^3) of the dataflow closure's fixed order for R = ceil(C / 128) pivot blocks:
@@ -179,7 +181,8 @@ SE_API int se_closure_schedule(int C, int lane_bits, int64_t work_bytes);
 
 /* 1 if the automatic schedule, as it is set now, tries the resident closure first for C
  * candidates with lane_bits (0: its first attempt, in 16-bit lanes) and work_bytes of workspace;
- * else 0. Host-only: it assumes a whole B200 and a stream that is not capturing. */
+ * else 0. Host-only: it assumes a whole B200, a stream that is not capturing, and no resident closure
+ * in flight on another stream. */
 SE_API int se_closure_resident(int C, int lane_bits, int64_t work_bytes);
 
 /* What the calling thread's last closure call (se_closure, se_closure_enqueue,

@@ -1,4 +1,5 @@
 // Error reporting, version and device information for the C ABI (include/se.h).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdarg>
@@ -14,6 +15,31 @@ namespace se {
 
 namespace {
 thread_local char g_last_error[1024] = {0};
+
+using CtxGetId = CUresult (*)(CUcontext, unsigned long long*);
+using CtxGetCurrent = CUresult (*)(CUcontext*);
+}  // namespace
+
+unsigned long long current_context_id() {
+    static CtxGetId get_id = nullptr;
+    static CtxGetCurrent get_current = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<CtxGetId>(p);
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<CtxGetCurrent>(p);
+        cudaGetLastError();
+    });
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (get_id && get_current && get_current(&ctx) == CUDA_SUCCESS && ctx && get_id(ctx, &id) == CUDA_SUCCESS)
+        return id;
+    return 0;
 }
 
 void set_error(const char* fmt, ...) {

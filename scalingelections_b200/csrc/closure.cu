@@ -1365,8 +1365,9 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
         if (se_status_t st = prepare_launches(lane_bits)) return st;
         for (;;) {
             bool ran = false;
+            resident::Hold hold(!sync);
             if (se_status_t st = resident::run(d_pref, ld_pref, C, d_out, ld_out, lb, base, lane_bits == 0, work,
-                                               work_bytes, s, &ran))
+                                               work_bytes, s, hold, &ran))
                 return st;
             if (!ran) break;
             g_last_schedule = SE_CLOSURE_RESIDENT;

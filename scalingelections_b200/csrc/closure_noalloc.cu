@@ -22,7 +22,6 @@
 // clears what must start at zero (its error word) and overwrites every cell of its working
 // matrix before reading it. Calls that overlap on the GPU, e.g. on two streams, race on the
 // array and must be serialised by the caller.
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -52,32 +51,6 @@ constexpr int kMaxDevices = 256;
 void* g_scratch_addr[kMaxDevices] = {};
 unsigned long long g_scratch_ctx[kMaxDevices] = {};
 
-using CtxGetId = CUresult (*)(CUcontext, unsigned long long*);
-using CtxGetCurrent = CUresult (*)(CUcontext*);
-
-// The current context's id (0 if the driver cannot say).
-unsigned long long current_context_id() {
-    static CtxGetId get_id = nullptr;
-    static CtxGetCurrent get_current = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<CtxGetId>(p);
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<CtxGetCurrent>(p);
-        cudaGetLastError();
-    });
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (get_id && get_current && get_current(&ctx) == CUDA_SUCCESS && ctx && get_id(ctx, &id) == CUDA_SUCCESS)
-        return id;
-    return 0;
-}
-
 // Device address of g_closure_scratch on the current device: looked up once per device (and
 // again only if that device's context has been replaced), with the device current.
 se_status_t scratch_address(void** out) {
@@ -86,7 +59,7 @@ se_status_t scratch_address(void** out) {
     SE_REQUIRE(dev >= 0 && dev < kMaxDevices, SE_ERR_INVALID, "device ordinal %d out of range", dev);
     std::lock_guard<std::mutex> lock(g_scratch_mutex);
     // Before the first runtime call on a device no context may be current (id 0): look up.
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = se::current_context_id();
     if (g_scratch_addr[dev] == nullptr || ctx == 0 || g_scratch_ctx[dev] != ctx) {
         void* p = nullptr;
         const cudaError_t e = cudaGetSymbolAddress(&p, g_closure_scratch);
@@ -96,7 +69,7 @@ se_status_t scratch_address(void** out) {
             return SE_ERR_CUDA;
         }
         g_scratch_addr[dev] = p;
-        g_scratch_ctx[dev] = current_context_id();  // the lookup made the device's context current
+        g_scratch_ctx[dev] = se::current_context_id();  // the lookup made the device's context current
     }
     *out = g_scratch_addr[dev];
     return SE_OK;

@@ -997,39 +997,89 @@ int64_t workspace_bytes(int C, int lane_bits) {
     return layout_of(C, lane_bits).total;
 }
 
-// Resident launches of one device run one after another: two of them in flight on different
-// streams could each hold part of the SMs and wait for the rest. Each launch records the device's
-// event, and a launch on another stream waits for it first.
-struct Order {
+// The resident launches of a device that may still be in flight, one entry per stream. Two of them that
+// do not fit the GPU together could each hold part of the SMs until both give way, so a launch that does
+// not fit beside those of other streams is not made: the closure then runs as launches. Nothing ever
+// waits for another stream. Streams and contexts are told apart by their ids: a handle may be
+// another thread's stream (cudaStreamPerThread), or a new stream in place of a destroyed one.
+struct Flight {
+    unsigned long long ctx = 0, stream = 0;
+    cudaEvent_t done = nullptr;  // of ctx; after the last launch of a call that only queues
+    int ctas = 0;                // of the largest launch not known to be done; 0: a free entry
+    int held = 0;                // calls that have not let go of the entry yet (Hold)
+};
+constexpr int kMaxFlights = 32;  // streams; with more in flight a closure runs as launches
+struct Flights {
     std::mutex m;
-    cudaEvent_t done = nullptr;
-    cudaStream_t last = nullptr;
+    Flight f[kMaxFlights];
 };
 constexpr int kMaxDevices = 64;
-Order& order_of(int dev) {
-    static Order orders[kMaxDevices];
-    return orders[dev];
+Flights& flights_of(int dev) {
+    static Flights all[kMaxDevices];
+    return all[dev];
 }
 
-// Makes s wait for the device's last resident launch, if that was on another stream. An event of
-// a context that has been reset is replaced: its launches are gone with it.
-se_status_t enter(Order& o, cudaStream_t s) {
-    if (o.done && o.last != s && cudaStreamWaitEvent(s, o.done, 0) != cudaSuccess) {
-        cudaGetLastError();
-        o.done = nullptr;
-    }
-    if (!o.done) SE_CUDA_TRY(cudaEventCreateWithFlags(&o.done, cudaEventDisableTiming));
-    return SE_OK;
+// An event may be asked for while another thread captures a stream.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Frees the entries whose event has come. A call that waits needs no event, and one whose launch fits
+// asks for none, so this costs only those that would have to run as launches.
+void drop_finished(Flights& F, unsigned long long ctx) {
+    RelaxedCapture relaxed;
+    for (Flight& x : F.f)
+        if (x.ctas && x.held == 0 && x.ctx == ctx) {
+            const cudaError_t e = x.done ? cudaEventQuery(x.done) : cudaSuccess;
+            if (e == cudaSuccess) x.ctas = 0;
+            else if (e == cudaErrorNotReady) cudaGetLastError();
+        }
 }
-se_status_t leave(Order& o, cudaStream_t s) {
-    if (cudaEventRecord(o.done, s) != cudaSuccess) {
-        cudaGetLastError();
-        o.done = nullptr;
-        SE_CUDA_TRY(cudaEventCreateWithFlags(&o.done, cudaEventDisableTiming));
-        SE_CUDA_TRY(cudaEventRecord(o.done, s));
+
+// The entry under which a launch of that many CTAs may be made, or null where it does not fit. A CTA
+// is counted as a whole SM, wherever it lands: CTAs that add up to no more than the SMs find room.
+Flight* admit(Flights& F, unsigned long long ctx, unsigned long long stream, int ctas, int sms, bool queued) {
+    std::lock_guard<std::mutex> lock(F.m);
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass) drop_finished(F, ctx);
+        Flight *mine = nullptr, *spare = nullptr;
+        int others = 0;
+        for (Flight& x : F.f) {
+            if (x.held == 0 && (x.ctas == 0 || x.ctx != ctx)) {  // another context's may be gone with it
+                if (!spare || x.ctas == 0) spare = &x;
+            } else if (x.ctx == ctx && x.stream == stream) {
+                mine = &x;
+            } else if (x.ctx == ctx) {
+                others += x.ctas;
+            }
+        }
+        Flight* x = mine ? mine : spare;
+        if (!x || (others && others + ctas > sms)) continue;
+        if (x != mine) {
+            if (x->ctx != ctx) x->done = nullptr;  // neither asked for nor reused
+            x->ctx = ctx;
+            x->stream = stream;
+            x->ctas = 0;
+        }
+        if (queued && !x->done && cudaEventCreateWithFlags(&x->done, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            x->done = nullptr;
+            return nullptr;
+        }
+        x->ctas = std::max(x->ctas, ctas);
+        ++x->held;
+        return x;
     }
-    o.last = s;
-    return SE_OK;
+    return nullptr;
+}
+
+Hold::~Hold() {
+    if (!flight) return;
+    std::lock_guard<std::mutex> lock(static_cast<Flights*>(flights)->m);
+    Flight& x = *static_cast<Flight*>(flight);
+    if (--x.held == 0 && !queued) x.ctas = 0;  // the call has waited for its stream
 }
 
 // The check-in's limit, of the calling thread's launches. Once the CTAs that there is room for spin, the
@@ -1042,7 +1092,7 @@ thread_local uint64_t g_wait_ns = kWaitNs;
 void set_wait_limit(uint64_t ns) { g_wait_ns = std::min(ns, 5 * kWaitNs); }
 
 se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_out, int lane_bits, uint32_t base,
-                bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, bool* ran) {
+                bool automatic, void* d_work, int64_t work_bytes, cudaStream_t s, Hold& hold, bool* ran) {
     *ran = false;
     if (C > max_candidates(lane_bits) || work_bytes < workspace_bytes(C, lane_bits)) return SE_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1078,7 +1128,6 @@ se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_
     P.start_ns = g_start_ns;
     P.wait_ns = g_wait_ns;
     P.polls = P.wait_ns ? 1u << 26 : 1u;
-    SE_CUDA_TRY(cudaMemsetAsync(work, 0, size_t(L.zero_bytes), s));
 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(ctas(*sh, L.NB)));
@@ -1091,16 +1140,21 @@ se_status_t run(const uint32_t* d, int64_t ld, int C, uint32_t* out, int64_t ld_
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void* args[] = {&P};
-    Order& o = order_of(dev);
-    std::lock_guard<std::mutex> lock(o.m);
-    if (se_status_t st = enter(o, s)) return st;
+    unsigned long long stream_id = 0;
+    SE_CUDA_TRY(cudaStreamGetId(s, &stream_id));
+    Flights& F = flights_of(dev);
+    Flight* flight = admit(F, current_context_id(), stream_id, int(cfg.gridDim.x), sms, hold.queued);
+    if (!flight) return SE_OK;
+    hold.flights = &F;
+    hold.flight = flight;
+    SE_CUDA_TRY(cudaMemsetAsync(work, 0, size_t(L.zero_bytes), s));
     const cudaError_t e = cudaLaunchKernelExC(&cfg, sh->fn, args);
     if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer CTAs fit than on a whole B200
         cudaGetLastError();
         return SE_OK;
     }
     SE_CUDA_TRY(e);
-    if (se_status_t st = leave(o, s)) return st;
+    if (hold.queued) SE_CUDA_TRY(cudaEventRecord(flight->done, s));
     *ran = true;
     return SE_OK;
 }

@@ -31,6 +31,10 @@ void clear_error();
 // records "cannot raise the shared-memory limit of <what>" and returns SE_ERR_CUDA.
 se_status_t raise_smem_limit(const void* fn, int bytes, const char* what);
 
+// The current context's id (0 if the driver cannot say). No id is used twice in a process, so what was
+// remembered of a device is known to be out of date after cudaDeviceReset.
+unsigned long long current_context_id();
+
 #define SE_CUDA_TRY(expr)                                                                     \
     do {                                                                                      \
         cudaError_t se_err_ = (expr);                                                         \
