@@ -417,7 +417,7 @@ SE_API se_status_t se_tally(const int32_t* d_ids, const int64_t* d_offsets, int6
                      void* stream);
 
 /* se_tally that also checks the ballot index as it reads it: d_offsets must start at 0, never
- * decrease and end at num_ids, else the call returns SE_ERR_INVALID (and d_out is undefined). No
+ * decrease and end at num_ids, else the call returns SE_ERR_INVALID and leaves d_out as it was. No
  * kernel follows an offset that breaks this. */
 SE_API se_status_t se_tally_checked(const int32_t* d_ids, int64_t num_ids, const int64_t* d_offsets,
                                     int64_t V, int C, uint32_t* d_out, int64_t ld_out, void* d_work,

@@ -287,7 +287,8 @@ def tally_workspace_bytes(num_voters: int, num_candidates: int) -> int:
 def tally_device(ids: torch.Tensor, offsets: torch.Tensor, num_candidates: int, *, out: torch.Tensor | None = None,
                  workspace: torch.Tensor | None = None) -> torch.Tensor:
     """Pairwise preference counts from CSR ballots on the device: ids int32 (concatenated
-    ballots, most preferred first), offsets int64 [V + 1]. Returns uint32 [C, C]."""
+    ballots, most preferred first), offsets int64 [V + 1]. Returns uint32 [C, C]. Offsets that do not
+    start at 0, decrease or do not end at len(ids) raise a ValueError and leave ``out`` as it was."""
     if ids.dtype != torch.int32 or offsets.dtype != torch.int64 or not ids.is_cuda or not offsets.is_cuda:
         raise TypeError("ids must be CUDA int32 and offsets CUDA int64")
     C = int(num_candidates)
@@ -303,8 +304,11 @@ def tally_device(ids: torch.Tensor, offsets: torch.Tensor, num_candidates: int, 
     with torch.cuda.device(ids.device):
         status = _lib.lib().se_tally_checked(ids.data_ptr(), ids.numel(), offsets.data_ptr(), V, C, out.data_ptr(),
                                              ldo, workspace.data_ptr(), need, _stream())
-    if status == _lib.SE_ERR_INVALID and "offsets must" in _lib.last_error():
-        raise ValueError(_lib.last_error())
+    if status == _lib.SE_ERR_INVALID and V > 0:
+        message = _lib.last_error()  # another refusal may have come before the kernels read the offsets
+        if bool((offsets[0] != 0) | (offsets[-1] != ids.numel()) | (offsets[1:] < offsets[:-1]).any()):
+            raise ValueError("offsets must start at 0, never decrease and end at len(ids)")
+        raise _lib.SchulzeError(status, message)
     check(status)
     return out
 

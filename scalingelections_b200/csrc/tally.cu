@@ -65,7 +65,8 @@ __device__ __forceinline__ void record_irregular(const Irregular& irr, int64_t v
 
 // Ballot v's span of ids. With num_ids >= 0 the offsets are checked as they are read: they must
 // start at 0, never decrease and end at num_ids. A ballot whose span breaks that is reported and
-// read as empty, so no kernel follows a bad bound; the check costs the tally no pass of its own.
+// read as empty, so no kernel follows a bad bound, and the kernels after the one that reads the
+// offsets leave the output alone; the check costs the tally no pass of its own.
 struct Span {
     int64_t beg, len;
     bool ok;
@@ -285,7 +286,9 @@ __device__ __forceinline__ int64_t range_start(const CountSplit& sp, int R, int6
 constexpr int kZeroParts = 8;
 
 __global__ void __launch_bounds__(256)
-    zero_tiles_kernel(uint32_t* __restrict__ out, int64_t ld_out, int C, int R, int64_t chunks, CountSplit sp) {
+    zero_tiles_kernel(uint32_t* __restrict__ out, int64_t ld_out, int C, int R, int64_t chunks, CountSplit sp,
+                      const uint32_t* __restrict__ err) {
+    if (*err == kErrOffsets) return;
     const int64_t b = int64_t(blockIdx.x) + 1, G = int64_t(gridDim.x) + 1;
     const int64_t u = range_start(sp, R, chunks, b, G), t = u / chunks;
     if (u % chunks == 0) return;
@@ -327,7 +330,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int chunks = int((V + kVC - 1) / kVC);
     const int64_t start = range_start(sp, R, chunks, cta, G);
     const int64_t in_rounds = sp.rounds * chunks;  // units in whole-tile rounds
-    const int64_t units = in_rounds + range_start(sp, R, chunks, cta + 1, G) - start;
+    // None where an earlier kernel has refused the offsets (this one only replaces a 0 in err).
+    const int64_t units = *err == kErrOffsets ? 0 : in_rounds + range_start(sp, R, chunks, cta + 1, G) - start;
     // Unit n of this CTA: its tile and chunk.
     auto locate = [&](int64_t n, int& I, int& J, int& ch) {
         const int64_t u = n < in_rounds ? n : start + (n - in_rounds);
@@ -507,10 +511,10 @@ template <typename Id>
 __global__ void __launch_bounds__(kIrrThreads)
     irregular_kernel(const Id* __restrict__ ids, const int64_t* __restrict__ offsets, int64_t id_base, int C,
                      const uint32_t* __restrict__ irr_n, const uint32_t* __restrict__ irr_list,
-                     uint32_t* __restrict__ out, int64_t ld_out) {
+                     const uint32_t* __restrict__ err, uint32_t* __restrict__ out, int64_t ld_out) {
     extern __shared__ uint32_t present[];
     const uint32_t n = *irr_n;
-    if (n == 0u) return;
+    if (n == 0u || *err == kErrOffsets) return;
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int64_t gw = int64_t(blockIdx.x) * warps + (threadIdx.x >> 5);
     const int64_t GW = int64_t(gridDim.x) * warps;
@@ -704,7 +708,7 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     const double cut_us = (double(above) + 0.8 * R) / double(grid) * full_us + 2 * 12.0 + 6.0;
     layout.whole = double((above + R + grid - 1) / grid) * (full_us + 3.0) <= cut_us;
     if (!accumulate && !layout.whole && grid > 1) {
-        zero_tiles_kernel<<<dim3(unsigned(grid - 1), kZeroParts), 256, 0, s>>>(d_out, ld_out, C, R, chunks, layout);
+        zero_tiles_kernel<<<dim3(unsigned(grid - 1), kZeroParts), 256, 0, s>>>(d_out, ld_out, C, R, chunks, layout, err);
         SE_CHECK_LAUNCH();
     }
     K.count<<<unsigned(grid), kThreads, bits_smem(B), s>>>(map, V, C, R, layout, d_out, ld_out, accumulate, irr.chunk,
@@ -718,19 +722,19 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
         if (se_status_t st = raise_smem_limit(reinterpret_cast<const void*>(fn), kIrrMaxSmem, "the irregular-ballot kernel"))
             return st;
         fn<<<irr_grid, kIrrThreads, irr_smem, s>>>(static_cast<const int32_t*>(d_ids), d_offsets, id_base, C, irr.n,
-                                                  irr.list, d_out, ld_out);
+                                                  irr.list, err, d_out, ld_out);
     } else if (id_bytes == 2) {
         auto fn = irregular_kernel<uint16_t>;
         if (se_status_t st = raise_smem_limit(reinterpret_cast<const void*>(fn), kIrrMaxSmem, "the irregular-ballot kernel"))
             return st;
         fn<<<irr_grid, kIrrThreads, irr_smem, s>>>(static_cast<const uint16_t*>(d_ids), d_offsets, id_base, C, irr.n,
-                                                  irr.list, d_out, ld_out);
+                                                  irr.list, err, d_out, ld_out);
     } else {
         auto fn = irregular_kernel<uint8_t>;
         if (se_status_t st = raise_smem_limit(reinterpret_cast<const void*>(fn), kIrrMaxSmem, "the irregular-ballot kernel"))
             return st;
         fn<<<irr_grid, kIrrThreads, irr_smem, s>>>(static_cast<const uint8_t*>(d_ids), d_offsets, id_base, C, irr.n,
-                                                  irr.list, d_out, ld_out);
+                                                  irr.list, err, d_out, ld_out);
     }
     SE_CHECK_LAUNCH();
     if (!check) return SE_OK;
