@@ -140,9 +140,8 @@ SE_API int64_t se_closure_workspace_bytes_flow(int C, int lane_bits, int tile);
 SE_API se_status_t se_closure_flow_task(uint32_t t, int R, int* kind, int* k, int* i, int* j);
 
 /* Process-wide schedule of se_closure (results are identical in every one):
- *   0  automatic (default): the resident closure where it applies (small C, see
- *      se_closure_workspace_bytes_flow), else by C from the variant table below; 1 where it
- *      has no entry;
+ *   0  automatic (default): by C from the variant table below, which starts with the resident
+ *      closure for small C (see se_closure_workspace_bytes_flow); 1 where it has no entry;
  *   1  round by round: pivot, panels and remainder launches per round, panels and pivots on
  *      the default micro-tile (8 x 8 words per thread), the next round's pivot closed by the
  *      first CTA of the remainder launch (with se_closure_workspace_bytes_flow() of workspace
@@ -167,8 +166,10 @@ SE_API se_status_t se_closure_flow_task(uint32_t t, int R, int* kind, int* k, in
 SE_API se_status_t se_closure_set_mode(int mode);
 
 /* The variant table of the automatic schedule: for C <= max_c[i] (the first i that holds) use
- * modes[i] (1 or 3 to 8); C above every entry uses 1. n <= 8; n = 0 clears it. The built-in
- * table, measured on B200, is {C <= 1024: 7, C <= 4096: 8, larger: 6}. An autotuner
+ * modes[i] (1, 3 to 8, or SE_CLOSURE_RESIDENT); C above every entry uses 1. An entry with
+ * SE_CLOSURE_RESIDENT is passed over, to the next that holds, wherever the resident closure does not
+ * apply; a table without one never runs it. n <= 8; n = 0 clears it. The built-in table, measured
+ * on B200, is {C <= 1536: resident, C <= 1024: 7, C <= 4096: 8, larger: 6}. An autotuner
  * measures the variants per size bucket and installs the winners (scalingelections_b200
  * autotune.tune_closure). No reference counterpart: the reference's tile_size argument picks
  * among its kernels' tile templates (scaling_elections.cu:895-901). */

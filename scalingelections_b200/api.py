@@ -156,7 +156,8 @@ _closure_mode = 0
 
 def set_closure_mode(mode: int) -> None:
     """The closure's schedule (same results in every one): 0 automatic by size (default; up to
-    C = 1536 with the full workspace one launch that keeps the matrix in registers),
+    C = 1536 with the full workspace one launch that keeps the matrix in registers, unless
+    set_closure_variants has set a table without it),
     1 round by round, 2 the dataflow form, 3 round by round with the panels on the wide
     micro-tile, 4 as 3 with each pivot tile closed by its own wide launch, 5 as 3 on two
     streams so the next round's chain overlaps the current remainder, 6 each round's
@@ -167,10 +168,10 @@ def set_closure_mode(mode: int) -> None:
     _closure_mode = int(mode)
 
 
-BUILTIN_CLOSURE_VARIANTS = ((1024, 7), (4096, 8), (1 << 20, 6))
+CLOSURE_RESIDENT = 9  # in a table and from last_closure_schedule(): the one-launch closure in registers
 
-
-CLOSURE_RESIDENT = 9  # last_closure_schedule(): the one-launch closure in registers
+BUILTIN_CLOSURE_VARIANTS = ((1536, CLOSURE_RESIDENT), (1024, 7), (4096, 8), (1 << 20, 6))
+_closure_variants: list[tuple[int, int]] = list(BUILTIN_CLOSURE_VARIANTS)  # what set_closure_variants last set
 
 
 def closure_schedule(num_candidates: int, lanes: int = LANES_U16, workspace_bytes: int | None = None) -> int:
@@ -200,15 +201,19 @@ def last_closure_schedule() -> int:
 
 
 def set_closure_variants(table: Sequence[tuple[int, int]]) -> None:
-    """The automatic schedule's table: (max_C, mode) pairs, first match wins, modes 1 or 3-8;
-    sizes above every entry run mode 1. An empty table clears it (every size then runs mode 1;
-    the library starts with the table measured on B200, {1024: 7, 4096: 8, 2**20: 6}).
-    autotune.tune_closure measures the modes per size bucket and installs its winners through
-    this."""
+    """The automatic schedule's table: (max_C, mode) pairs, first match wins, modes 1, 3-8 or
+    CLOSURE_RESIDENT, which is passed over where the one-launch closure does not apply and which a
+    table without it never runs; sizes above every entry run mode 1. An empty table clears it
+    (every size then runs mode 1); the library starts with BUILTIN_CLOSURE_VARIANTS, measured on
+    B200. autotune.tune_closure measures the modes per size bucket and installs its winners
+    through this."""
+    global _closure_variants
+    table = [(int(c), int(m)) for c, m in table]
     n = len(table)
-    max_c = (ctypes.c_int * max(n, 1))(*[int(c) for c, _ in table])
-    modes = (ctypes.c_int * max(n, 1))(*[int(m) for _, m in table])
+    max_c = (ctypes.c_int * max(n, 1))(*[c for c, _ in table])
+    modes = (ctypes.c_int * max(n, 1))(*[m for _, m in table])
     check(_lib.lib().se_closure_set_variant_table(max_c, modes, n))
+    _closure_variants = table
 
 
 def strongest_paths_device(preferences: torch.Tensor, *, lanes: int = LANES_AUTO, out: torch.Tensor | None = None,

@@ -1,8 +1,9 @@
 """Autotuners for the batched closure and for the single-election closure.
 
-tune_closure: for each size bucket of the single-election closure it times the round-by-round
-schedules on a sample matrix and installs the fastest per bucket in the library's variant
-table (se_closure_set_variant_table), which the automatic schedule reads:
+tune_closure: for each size bucket of the single-election closure it times the one-launch
+closure (mode 9, where the size allows it) and the schedules of launches on a sample matrix and
+installs the fastest per bucket in the library's variant table (se_closure_set_variant_table),
+which the automatic schedule reads:
   1  panels and pivots on the default micro-tile (8 x 8 words per thread, four warps in
      16-bit lanes), the next pivot fused into the remainder launch;
   3  panels on the wide micro-tile (8 x 4 words per thread, eight warps);
@@ -133,8 +134,8 @@ def tune(V: int = 100000, per_bucket: int = 48, reps: int = 3, seed: int = 0, pa
     return table
 
 
-CLOSURE_BUCKETS = [1024, 2048, 3072, 4096, 6144, 8192, 12288]  # upper bounds of the size buckets
-CLOSURE_MODES = (1, 3, 4, 5, 6, 7, 8)
+CLOSURE_BUCKETS = [1024, 1536, 2048, 3072, 4096, 6144, 8192, 12288]  # upper bounds of the size buckets
+CLOSURE_MODES = (9, 1, 3, 4, 5, 6, 7, 8)
 
 
 def tune_closure(sizes: Sequence[int] | None = None, reps: int = 5, V: int = 4096, seed: int = 0,
@@ -142,22 +143,28 @@ def tune_closure(sizes: Sequence[int] | None = None, reps: int = 5, V: int = 409
     """Times the closure schedules CLOSURE_MODES at one size per bucket (the bucket's upper
     bound by default; 16-bit lanes, a random tally of V ballots) and returns
     {"sizes": {C: {mode: ms}}, "table": [(max_C, best mode), ...]}; installs the table in the
-    library when `install`. Buckets above the last size keep mode 1."""
+    library when `install`, else leaves the one that set_closure_variants set. A call that cannot
+    take the one-launch closure where that won runs the next bucket's schedule. Buckets above the
+    last size keep mode 1."""
     from . import api
 
     device = device or torch.device("cuda", torch.cuda.current_device())
     sizes = list(sizes or CLOSURE_BUCKETS)
     out = {"sizes": {}, "table": []}
     s = torch.cuda.current_stream()
+    before = api._closure_variants
     try:
         for n, C in enumerate(sizes):
+            api.set_closure_variants([(int(C), api.CLOSURE_RESIDENT)])
             d = _sample_batch(C, C, 1, V, seed + n, device)[0]
             work = torch.empty(api.closure_workspace_bytes(C, LANES_U16, dataflow=True), dtype=torch.uint8,
                                device=device)
             res = torch.empty_like(d)
             times = {}
             for mode in CLOSURE_MODES:
-                api.set_closure_mode(mode)
+                api.set_closure_mode(0 if mode == api.CLOSURE_RESIDENT else mode)
+                if mode == api.CLOSURE_RESIDENT and not api.closure_is_resident(C):
+                    continue
                 api.strongest_paths_device(d, lanes=LANES_U16, out=res, workspace=work)
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record(s)
@@ -171,6 +178,7 @@ def tune_closure(sizes: Sequence[int] | None = None, reps: int = 5, V: int = 409
             del d, work, res
     finally:
         api.set_closure_mode(0)
+        api.set_closure_variants(before)
     if install:
         api.set_closure_variants(out["table"])
     return out

@@ -752,8 +752,8 @@ layout plan(int C, int lane_bits) {
 }
 
 // Closure schedules (se_closure_set_mode):
-//   0  automatic: the resident closure (closure_resident.cu) where the matrix and the workspace fit
-//      it, else by C, from the variant table (se_closure_set_variant_table), else 1;
+//   0  automatic: by C, from the variant table (se_closure_set_variant_table), whose built-in
+//      entries put the resident closure (closure_resident.cu) first, else 1;
 //   1  round by round, panels and pivots with the default micro-tile (8 x 8 words, 128
 //      threads in 16-bit lanes), the next round's pivot fused into the remainder launch;
 //   2  dataflow: one persistent grid (needs se_closure_workspace_bytes_flow() of workspace);
@@ -780,17 +780,24 @@ std::atomic<int> g_closure_mode{0};
 // (16-bit lanes, ms per closure, 5 closures each; modes 3 / 6 / 7 / 8): C = 1024 0.441 / 0.473
 // / 0.432 / 0.443, C = 2048 0.962 / 0.976 / 0.974 / 0.947, C = 3072 1.855 / 1.759 / 1.865 /
 // 1.750, C = 4096 3.783 / 3.398 / 4.200 / 3.397, C = 5120 6.870 / 6.392 / 7.611 / 6.452, C =
-// 6144 10.85 / 10.84 / 11.45 / 11.08. The table is within 2.2 % of the fastest mode at each.
+// 6144 10.85 / 10.84 / 11.45 / 11.08. The table is within 2.2 % of the fastest mode at each. The first
+// entry is the resident closure's, measured in closure_resident.cu; an entry with it is passed over where
+// it does not apply (size in these lanes, workspace, a capturing stream, SMs held by others).
 constexpr int kMaxVariants = 8;
 std::mutex g_variant_mutex;
-int g_variant_n = 3;
-int g_variant_max_c[kMaxVariants] = {1024, 4096, 1 << 20};
-int g_variant_mode[kMaxVariants] = {7, 8, 6};
+int g_variant_n = 4;
+int g_variant_max_c[kMaxVariants] = {resident::max_candidates(16), 1024, 4096, 1 << 20};
+int g_variant_mode[kMaxVariants] = {SE_CLOSURE_RESIDENT, 7, 8, 6};
 
-int automatic_mode(int C) {
+// The table's schedule of launches for C, and whether the resident closure stands before it.
+int automatic_mode(int C, bool* resident = nullptr) {
     std::lock_guard<std::mutex> lock(g_variant_mutex);
-    for (int i = 0; i < g_variant_n; ++i)
-        if (C <= g_variant_max_c[i]) return g_variant_mode[i];
+    if (resident) *resident = false;
+    for (int i = 0; i < g_variant_n; ++i) {
+        if (C > g_variant_max_c[i]) continue;
+        if (g_variant_mode[i] != SE_CLOSURE_RESIDENT) return g_variant_mode[i];
+        if (resident) *resident = true;
+    }
     return 1;
 }
 
@@ -812,7 +819,9 @@ int schedule_in_lanes(int mode, int lane_bits) {
 
 // Whether the automatic schedule tries the resident closure first.
 bool resident_first(int C, int lane_bits, int64_t work_bytes) {
-    return g_closure_mode.load() == 0 && C <= resident::max_candidates(lane_bits) &&
+    bool named = false;
+    automatic_mode(C, &named);
+    return named && g_closure_mode.load() == 0 && C <= resident::max_candidates(lane_bits) &&
            work_bytes >= resident::workspace_bytes(C, lane_bits);
 }
 
@@ -1354,13 +1363,14 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
     int lb = lane_bits == 0 ? 16 : lane_bits;
     uint32_t base = value_offset;
     int mode = mode_override >= 0 ? mode_override : g_closure_mode.load();
-    const bool automatic = mode == 0;
+    bool resident_named = false;
+    if (mode == 0) automatic_mode(C, &resident_named);
     // Matrices that fit the SMs' register files close in one launch (closure_resident.cu): 1.4 to
     // 2.1 times faster than the launches below at every size that it takes (its shapes' table).
     // That launch may give way where other kernels hold the SMs that it needs. A call that waits
     // then runs the launches; one that only queues has queued gated launches behind it, so it needs
     // room for them, and a second pivot block for that form to apply.
-    if (automatic && phase_ms == nullptr &&
+    if (resident_named && phase_ms == nullptr &&
         (sync || resident::single_cta(C) || (C > kT && work_bytes >= plan(C, lb).flow_total))) {
         if (se_status_t st = prepare_launches(lane_bits)) return st;
         for (;;) {
@@ -1549,8 +1559,8 @@ extern "C" se_status_t se_closure_set_variant_table(const int* max_c, const int*
         SE_REQUIRE(n >= 0 && n <= kMaxVariants, SE_ERR_INVALID, "at most %d table entries", kMaxVariants);
         SE_REQUIRE(n == 0 || (max_c && modes), SE_ERR_INVALID, "null table");
         for (int i = 0; i < n; ++i)
-            SE_REQUIRE(modes[i] == 1 || (modes[i] >= 3 && modes[i] <= 8), SE_ERR_INVALID,
-                       "table modes must be 1 or 3 to 8 (got %d)", modes[i]);
+            SE_REQUIRE(modes[i] == 1 || (modes[i] >= 3 && modes[i] <= SE_CLOSURE_RESIDENT), SE_ERR_INVALID,
+                       "table modes must be 1 or 3 to 9 (got %d)", modes[i]);
         std::lock_guard<std::mutex> lock(g_variant_mutex);
         for (int i = 0; i < n; ++i) {
             g_variant_max_c[i] = max_c[i];
