@@ -60,16 +60,17 @@ se_status_t raise_smem_limit(const void* fn, int bytes, const char* what) {
     }
     return host_guard([&]() -> se_status_t {  // the cache's insert can throw std::bad_alloc
         static std::mutex m;
-        static std::set<std::tuple<const void*, int, int>> done;
+        static std::set<std::tuple<const void*, int, unsigned long long, int>> done;  // a new context has none
         std::lock_guard<std::mutex> lock(m);
-        if (done.count({fn, dev, bytes})) return SE_OK;
+        const unsigned long long ctx = current_context_id();
+        if (done.count({fn, dev, ctx, bytes})) return SE_OK;
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error("cannot raise the shared-memory limit of %s: %s", what, cudaGetErrorString(e));
             return SE_ERR_CUDA;
         }
-        done.insert({fn, dev, bytes});
+        done.insert({fn, dev, current_context_id(), bytes});
         return SE_OK;
     });
 }

@@ -913,14 +913,16 @@ se_status_t side_stream(cudaStream_t* out) {
     constexpr int kMaxDev = 64;
     static std::mutex m;
     static cudaStream_t streams[kMaxDev] = {};
+    static unsigned long long contexts[kMaxDev] = {};  // whose they are: a reset takes them along
     int dev = 0;
     SE_CUDA_TRY(cudaGetDevice(&dev));
     SE_REQUIRE(dev >= 0 && dev < kMaxDev, SE_ERR_INVALID, "device ordinal %d out of range", dev);
     std::lock_guard<std::mutex> lock(m);
-    if (!streams[dev]) {
+    if (!streams[dev] || contexts[dev] != current_context_id()) {  // the calls before made the context current
         int least = 0, greatest = 0;
         SE_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         SE_CUDA_TRY(cudaStreamCreateWithPriority(&streams[dev], cudaStreamNonBlocking, least));
+        contexts[dev] = current_context_id();
     }
     *out = streams[dev];
     return SE_OK;
@@ -1306,17 +1308,15 @@ se_status_t report_flags(const uint32_t* flags);
 
 // A call outside a capture also readies the launches, so that a later call may be captured.
 se_status_t prepare_launches(int lane_bits) {
-    static std::atomic<uint64_t> ready[2];
+    constexpr int kDevices = 64;
+    static std::atomic<unsigned long long> ready[2][kDevices];  // the id of the context that is (0: none yet)
     int dev = 0;
     SE_CUDA_TRY(cudaGetDevice(&dev));
-    const uint64_t bit = 1ull << (dev & 63);
-    if (lane_bits != 32 && !(ready[0].load() & bit)) {
-        if (se_status_t st = set_smem_limits<16>()) return st;
-        ready[0].fetch_or(bit);
-    }
-    if (lane_bits != 16 && !(ready[1].load() & bit)) {
-        if (se_status_t st = set_smem_limits<32>()) return st;
-        ready[1].fetch_or(bit);
+    const unsigned long long id = current_context_id();
+    for (int lb = 0; lb < 2; ++lb) {
+        if (lane_bits == (lb ? 16 : 32) || (id && dev < kDevices && ready[lb][dev].load() == id)) continue;
+        if (se_status_t st = lb ? set_smem_limits<32>() : set_smem_limits<16>()) return st;
+        if (dev < kDevices) ready[lb][dev].store(current_context_id());
     }
     return SE_OK;
 }
