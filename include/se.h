@@ -244,7 +244,9 @@ SE_API se_status_t se_closure_noalloc(const uint32_t* d_pref, int64_t ld_pref, i
  *   se_batch_prepare           builds the task queues and tensor maps and uploads them into
  *                              d_work (synchronous copies); fills the caller's plan.
  *                              order: 0 = small elections after the tiled ones, 1 = before.
- *                              ctas_per_sm: persistent CTAs per SM (0 = as many as fit).
+ *                              ctas_per_sm: persistent CTAs per SM, at most as many as fit (a
+ *                              large number: as many as fit). 0: per queue, one where its tasks
+ *                              are few for its largest election's chain, else as many as fit.
  *   se_batch_run               enqueues one whole batch on `stream` (asynchronous, no host
  *                              synchronisation, capturable).
  *   se_batch_graph_build       captures se_batch_run into a CUDA graph held by the plan;
@@ -294,6 +296,8 @@ SE_API se_status_t se_batch_profile(const se_batch_plan_t* plan, double* busy_ms
 /* Number of tasks in queue 0 (16-bit lanes), 1 (32-bit lanes) or 2 (16-bit lanes on the wide
  * micro-tile) of a prepared plan. */
 SE_API int64_t se_batch_task_count(const se_batch_plan_t* plan, int queue);
+/* CTAs of that queue's persistent launch. */
+SE_API int se_batch_cta_count(const se_batch_plan_t* plan, int queue);
 
 /* ---------------------------------------------------------------------------------------
  * Serving engine (no reference counterpart): continuous batching of whole elections (tally,

@@ -192,7 +192,7 @@ def load(path: Path | None = None) -> dict | None:
 def choose(table: dict | None, Cs: Sequence[int], Vs: Sequence[int]) -> tuple[list, int, int]:
     """(lanes per election, order, ctas_per_sm) for a batch: per-bucket lane modes from the
     table (falling back to the widest legal 16-bit window), and the table's launch settings
-    (0 CTAs per SM, i.e. as many as fit, without a table)."""
+    (without a table 0 CTAs per SM: each launch by the library's rule)."""
     lanes = []
     for C, V in zip(Cs, Vs):
         entry = (table or {}).get("buckets", {}).get(str(bucket_of(int(C))))

@@ -36,9 +36,10 @@ class BatchedElections:
     read for the whole batch). micro_tiles: per election, 8 (the default 8 x 8-word micro-tile)
     or 4 (the wide 8 x 4-word one, 256-thread CTAs; 16-bit lanes), run as separate persistent
     launches; None is 8 everywhere. order: 0 runs small elections (C <= 128) after the tiled
-    ones, 1 before them. ctas_per_sm: persistent CTAs per SM (0 = as many as fit). An autotuned
-    table (scalingelections_b200.autotune) supplies lanes, micro-tiles, order and ctas_per_sm
-    per size bucket. The batch keeps references to every buffer it uses."""
+    ones, 1 before them. ctas_per_sm: persistent CTAs per SM, at most as many as fit (0: each of the
+    persistent launches takes one where its tasks are few for its largest election's chain, else as
+    many as fit). An autotuned table (scalingelections_b200.autotune) supplies lanes, micro-tiles,
+    order and ctas_per_sm per size bucket. The batch keeps references to every buffer it uses."""
 
     def __init__(self, preferences: Sequence[torch.Tensor], lanes: Sequence | None = None, *,
                  ranking: bool = True, order: int = 0, ctas_per_sm: int = 0,
@@ -102,6 +103,11 @@ class BatchedElections:
         the wide micro-tile."""
         L = _lib.lib()
         return tuple(L.se_batch_task_count(ctypes.byref(self.plan), q) for q in range(3))
+
+    def cta_counts(self) -> tuple[int, int, int]:
+        """CTAs of the three persistent launches, in the same order."""
+        L = _lib.lib()
+        return tuple(L.se_batch_cta_count(ctypes.byref(self.plan), q) for q in range(3))
 
     def run(self) -> None:
         """Enqueue the whole batch on the current stream (asynchronous)."""

@@ -695,6 +695,24 @@ extern "C" int64_t se_batch_workspace_bytes(int n, const se_election_t* election
     return total;
 }
 
+// Whether a queue's persistent launch takes one CTA per SM, not as many as fit, where the caller leaves it
+// open. The queues run one after another, so each has a chain and tasks of its own. Two CTAs per SM get
+// through more tasks (3.4 us less per tile task and SM on the 8 x 8 micro-tile, 2.8 on the wide one, about
+// 12 per small election), but a round of the largest election's chain (panels, its first remainder tile
+// with the next pivot) takes longer beside a second CTA: by 17 and 22 us, both fitted. So a queue whose
+// tasks are few for its chain takes one. One B200, us with one / two CTAs per SM, sizes log-uniform:
+//   8 x 8   20 elections up to C = 2048 1442 / 1567, 40 1938 / 1895, 100 3749 / 3374; 20 up to C = 700
+//           400 / 490, 100 447 / 524, 300 818 / 820; 1000 up to C = 300 560 / 494
+//   wide    4 of 129 to 1800 1063 / 1289; 20 of 129 to 2048 1737 / 1845, 40 3138 / 3023, 100 5969 / 5275;
+//           20 of 129 to 700 381 / 469, 100 733 / 803, 300 1721 / 1518; 1000 of 129 to 300 1356 / 1084
+// Next to the line it can be 5 % off (4 of 1700 to 1800 on 8 x 8: 1609 / 1691, and it takes two). 32-bit
+// lanes fit one CTA per SM either way. Mixed, us with one / two for all, and by queue: 20 up to C = 2048 in
+// 16-bit and 20 in 32-bit lanes 3408 / 3548, 3431 (one rule over all queues took two).
+static bool one_cta_per_sm(int queue, int rounds, uint32_t tasks, uint32_t small, int sms) {
+    const double gain = 12.0 * small + (queue == 2 ? 2.8 : 3.4) * (double(tasks) - small);
+    return rounds > 1 && gain < double(rounds) * (queue == 2 ? 22.0 : 17.0) * double(sms);
+}
+
 // The batch's host-side planning: sizes, the task queues and their dependency prefixes, all in
 // host vectors that are filled before anything is written to the device.
 static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_work, int64_t work_bytes, int order,
@@ -754,14 +772,18 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
     // Task queues. Largest elections first inside every step.
     std::vector<int32_t> order_big(big);
     std::stable_sort(order_big.begin(), order_big.end(), [&](int a, int b) { return host[a].R > host[b].R; });
-    int Rmax = 1;
-    for (int e : big) Rmax = std::max(Rmax, host[e].R);
+    int Rmax = 1, rmax[3] = {1, 1, 1};  // of all, and per queue
+    for (int e : big) {
+        rmax[z.queue[e]] = std::max(rmax[z.queue[e]], host[e].R);
+        Rmax = std::max(Rmax, host[e].R);
+    }
     std::vector<uint64_t> q[3];
     std::vector<uint64_t> small[2];
     for (int e = 0; e < n; ++e)
         if (host[e].R == 1) small[z.queue[e]].push_back(pack_task(e, kSmall, 0, 0, 0));
     if (order == 1)  // small elections first
         for (int l = 0; l < 2; ++l) q[l].insert(q[l].end(), small[l].begin(), small[l].end());
+    const uint32_t nsmall[3] = {uint32_t(small[0].size()), uint32_t(small[1].size()), 0u};
     for (int k = 0; k < Rmax; ++k) {
         if (k == 0)
             for (int e : order_big) q[z.queue[e]].push_back(pack_task(e, kPivot, 0, 0, 0));
@@ -847,25 +869,12 @@ static se_status_t batch_prepare_impl(int n, const se_election_t* el, void* d_wo
     const int occ16 = occupancy<16>(), occ32 = occupancy<32>(), occ16w = occupancy<16, 4>();
     SE_REQUIRE(occ16 >= 1 && occ32 >= 1 && occ16w >= 1, SE_ERR_CUDA, "batched closure kernel cannot be resident");
     SE_REQUIRE(ctas_per_sm >= 0, SE_ERR_INVALID, "ctas_per_sm must be >= 0");
-    // Two CTAs per SM finish a tile task every 12.6 us and SM, one CTA every 16 us, but a round of
-    // the largest election's chain (panels, its first remainder tile with the next pivot) takes
-    // longer beside a second CTA. So a batch whose tasks are few for its chain takes one CTA per SM:
-    // tasks * 3.4 us / SMs < rounds * 17 us, with the 17 fitted (a small election's task is about
-    // 12 us the shorter for a second CTA, a 32-bit tile's about 7). One B200, us with one / two CTAs
-    // per SM, sizes log-uniform: 20 elections up to C = 2048 1442 / 1567, 40 1938 / 1895, 100 3749 /
-    // 3374; 20 up to C = 700 400 / 490, 100 447 / 524, 300 818 / 820; 1000 up to C = 300 560 / 494.
-    if (ctas_per_sm == 0 && Rmax > 1) {
-        const double nsmall = double(n) - double(big.size());
-        const double gain = 12.0 * nsmall + 3.4 * (double(P.ntasks[0]) + double(P.ntasks[2]) - nsmall) +
-                            7.0 * double(P.ntasks[1]);
-        if (gain < double(Rmax) * 17.0 * double(sms)) ctas_per_sm = 1;
+    const int occ[3] = {occ16, occ32, occ16w};
+    for (int l = 0; l < 3; ++l) {
+        int per = ctas_per_sm > 0 ? std::min(occ[l], ctas_per_sm) : occ[l];
+        if (ctas_per_sm == 0 && one_cta_per_sm(l, rmax[l], P.ntasks[l], nsmall[l], sms)) per = 1;
+        P.grid[l] = int(std::min<int64_t>(P.ntasks[l], int64_t(sms) * per));
     }
-    const int per16 = ctas_per_sm > 0 ? std::min(occ16, ctas_per_sm) : occ16;
-    const int per32 = ctas_per_sm > 0 ? std::min(occ32, ctas_per_sm) : occ32;
-    const int per16w = ctas_per_sm > 0 ? std::min(occ16w, ctas_per_sm) : occ16w;
-    P.grid[0] = int(std::min<int64_t>(P.ntasks[0], int64_t(sms) * per16));
-    P.grid[1] = int(std::min<int64_t>(P.ntasks[1], int64_t(sms) * per32));
-    P.grid[2] = int(std::min<int64_t>(P.ntasks[2], int64_t(sms) * per16w));
     P.graph = nullptr;
     P.dep_wait_ns = kDepWaitNs;
     std::memcpy(plan_out, &P, sizeof(P));
@@ -984,4 +993,11 @@ extern "C" int64_t se_batch_task_count(const se_batch_plan_t* plan, int queue) {
     Plan P;
     std::memcpy(&P, plan, sizeof(P));
     return P.ntasks[queue];
+}
+
+extern "C" int se_batch_cta_count(const se_batch_plan_t* plan, int queue) {
+    if (!plan || queue < 0 || queue > 2) return -1;
+    Plan P;
+    std::memcpy(&P, plan, sizeof(P));
+    return P.grid[queue];
 }
