@@ -49,13 +49,15 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
 
 # Pageable host matrices reach the device through two pinned chunks: while one chunk's copy
 # to the device runs, host threads fill the other (NumPy releases the GIL for large copies). From
-# two chunks up this beats the driver's own staging (16 host threads, ms staged / driver: 36 MB 2.1 /
-# 1.8, 67 MB 2.8 / 5.1, 1074 MB 22.7 / 96); chunks of 16 MB pay more for their hand-over (3.5 ms at
-# 67 MB, 27 at 1074), ones of 64 MB overlap less (26 ms). One matrix at a time goes through them.
+# two chunks up, well past where this starts to beat the driver's own staging (16 host threads, ms
+# staged / driver: 24 MiB 2.0 / 1.5, 36 2.6 / 2.6, 48 2.9 / 4.1, 64 3.9 / 5.4, 128 6.5 / 11.9, 1024
+# 22.7 / 96); chunks of 16 MB pay more for their hand-over (3.5 ms at 67 MB, 27 at 1074), ones of
+# 64 MB overlap less (26 ms). One matrix at a time goes through a device's chunks.
 _STAGE_CHUNK = 32 << 20
 _STAGE_THREADS = 8
 _stage_state: dict = {}
-_stage_lock = threading.Lock()
+_stage_locks: dict = {}  # one per device
+_stage_guard = threading.Lock()  # of the table of locks
 
 
 def _stage_to_device(a: np.ndarray, dev) -> torch.Tensor:
@@ -63,7 +65,9 @@ def _stage_to_device(a: np.ndarray, dev) -> torch.Tensor:
     src = a.reshape(-1).view(np.uint8)
     n = src.size
     out = torch.empty(n, dtype=torch.uint8, device=dev)
-    with _stage_lock:
+    with _stage_guard:
+        lock = _stage_locks.setdefault(dev, threading.Lock())
+    with lock:
         _stage_locked(src, out, n, dev)
     return out
 
