@@ -47,6 +47,8 @@ __device__ __forceinline__ uint4 ldg4(const uint32_t* p) { return __ldg(reinterp
 // 16 bytes apart, each of which touches every sector of the row piece; there the thread's columns are
 // cx, cx + 16, cx + 32 and cx + 48 instead, so that a half warp's load is 64 contiguous bytes, and
 // row r's cells move by 2 * (r & 15) in the shared tile. C = 10007 on a B200: se_rank 99.9 -> 97.6 us.
+// The form of the edge branch below decides the registers of the whole kernel: with its four columns
+// worked out beforehand the wide kernel spilled (C = 8192 / 16384 59.5 / 189.8 us, so 57.7 / 184.7).
 template <bool WIDE> __device__ __forceinline__ int col_at(int cx, int q) { return WIDE ? 4 * cx + q : cx + 16 * q; }
 
 // Loads the thread's 4 x 4 cells of S[I][J] (a) and of S[J][I] at the same positions (b).
@@ -75,12 +77,13 @@ __device__ __forceinline__ void load_pair(const uint32_t* __restrict__ S, int64_
         }
     } else {
         auto at = [&](int r, int c) -> uint32_t { return (r < C && c < C) ? __ldg(S + int64_t(r) * ld + c) : 0u; };
-        const int c0 = col_at<WIDE>(cx, 0), c1 = col_at<WIDE>(cx, 1), c2 = col_at<WIDE>(cx, 2), c3 = col_at<WIDE>(cx, 3);
+        constexpr int kStep = WIDE ? 1 : 16;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-            const int ra = i0 + ry + 16 * p, rb = j0 + ry + 16 * p;
-            a[p] = make_uint4(at(ra, j0 + c0), at(ra, j0 + c1), at(ra, j0 + c2), at(ra, j0 + c3));
-            b[p] = make_uint4(at(rb, i0 + c0), at(rb, i0 + c1), at(rb, i0 + c2), at(rb, i0 + c3));
+            const int ra = i0 + ry + 16 * p, ca = j0 + (WIDE ? 4 : 1) * cx;
+            const int rb = j0 + ry + 16 * p, cb = i0 + (WIDE ? 4 : 1) * cx;
+            a[p] = make_uint4(at(ra, ca), at(ra, ca + kStep), at(ra, ca + 2 * kStep), at(ra, ca + 3 * kStep));
+            b[p] = make_uint4(at(rb, cb), at(rb, cb + kStep), at(rb, cb + 2 * kStep), at(rb, cb + 3 * kStep));
         }
     }
 }
