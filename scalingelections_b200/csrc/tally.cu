@@ -250,10 +250,13 @@ inline size_t bits_smem(int B) { return size_t(kBitStages) * 2 * B * kTile * 4 +
 // takes the whole tiles b, b + G, .. of the first `rounds` * G, all above the diagonal. The rest
 // is laid end to end as a line of (tile, 32-voter chunk) units and cut into G equal ranges, where
 // a unit above the diagonal weighs 5 and a diagonal one 4 (count_bits_kernel leaves out warps
-// there; the count of C = 1000, V = 60000 takes 724 us so, 755 with 4 and 3, 769 with equal
-// weights). A range ends anywhere inside a tile; such a tile's counts arrive as atomic adds.
-// `whole` moves the ends to tile ends. So no SM waits for a last partial wave, and a CTA has at
-// most two split tiles to add, however many voters there are.
+// there). se_tally, us, with weights 1 : 1 / 4 : 3 / 5 : 4 / 6 : 5: C = 256, V = 100000 212 / 208 /
+// 205 / 211; C = 500, V = 100000 508 / 483 / 484 / 489; C = 1000, V = 60000 914 / 912 / 886 / 894; C =
+// 1500, V = 30000 1028 / 1052 / 1006 / 1017; C = 2000, V = 20000 1224 / 1273 / 1212 / 1214; C = 3000,
+// V = 8000 1192 / 1190 / 1181 / 1166; 1 % or less between them from C = 4096 on. A range ends anywhere
+// inside a tile; such a tile's counts arrive as atomic adds. `whole` moves the ends to tile ends. So
+// no SM waits for a last partial wave, and a CTA has at most two split tiles to add, however many
+// voters there are.
 struct CountSplit {
     int64_t rounds;
     bool whole;
@@ -736,8 +739,11 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     // come out even, then the rest of the tiles cut into equal ranges (CountSplit). Cutting pays
     // when the wait for the last whole tiles is longer than what it adds: an output by atomic adds
     // at each end of a range and the zeroing before it. Costs in microseconds, measured on B200:
-    // counting 0.15 per 32-voter chunk and plane-plus-two, output 12 (atomic) or 3 (stores) per
-    // tile, zeroing 6.
+    // counting 0.15 per 32-voter chunk and plane-plus-two, a whole tile's output 3, cutting 27 where
+    // counts are added to out and 39 where it is zeroed first. Whole / cut, us: C = 2048, V = 3000
+    // 235 / 256, 5000 365 / 378, 7000 496 / 490, adding 238 / 248, 365 / 364, 494 / 481; C = 1900, V =
+    // 700 99 / 119, 2500 201 / 204, adding 101 / 111, 201 / 196; C = 4000, V = 500 191 / 207, 1500 451 / 436;
+    // C = 8000, V = 800 861 / 865, adding 862 / 857; C = 1000, V = 1500 128 / 104.
     int sms = 0, dev = 0;
     SE_CUDA_TRY(cudaGetDevice(&dev));
     SE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -747,7 +753,7 @@ se_status_t tally_impl(const void* d_ids, int id_bytes, const int64_t* d_offsets
     const double full_us = 0.15 * double(chunks) * double(B + 2);
     CountSplit layout{tiles_above(R) / grid, false};
     const int64_t above = tiles_above(R) - layout.rounds * grid;
-    const double cut_us = (double(above) + 0.8 * R) / double(grid) * full_us + 2 * 12.0 + 6.0;
+    const double cut_us = (double(above) + 0.8 * R) / double(grid) * full_us + (accumulate ? 27.0 : 39.0);
     layout.whole = double((above + R + grid - 1) / grid) * (full_us + 3.0) <= cut_us;
     if (!accumulate && !layout.whole && grid > 1) {
         zero_tiles_kernel<<<dim3(unsigned(grid - 1), kZeroParts), 256, 0, s>>>(d_out, ld_out, C, R, chunks, layout, err);
