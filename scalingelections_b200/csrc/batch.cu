@@ -159,16 +159,19 @@ __global__ void __launch_bounds__(tile_threads<LB, NQ>(), NQ == 4 ? 2 : 1)
             if constexpr (NQ == 8) run_small<LB>(E, smem, rowbuf, colbuf, s_wins, &hdr->err);
             else ok = false;  // the host never queues one here
         } else {
-            int pivot = type == kPivot ? int(k) : -1;
-            if (type != kPivot) {
+            // Two call sites: with one for both, whose tile is picked beforehand, the closing of the pivot
+            // took 1 to 2 us longer (us, one / two sites, one CTA per SM: 10 elections of 250 candidates
+            // 157.6 / 154.4, 60 of 500 586 / 579; two per SM: 300 of 200 356 / 349, 300 of 300 868 / 864).
+            if (type == kPivot) {
+                run_pivot<LB, NQ>(E, int(k), rowbuf, colbuf);
+            } else {
                 const int kind = type == kRow ? kTileRow : (type == kCol ? kTileCol : kTileRem);
                 ok = run_tile<LB, true, NQ>(E, &E, kind, int(k), int(i), int(j), smem, bars, par_a, par_b);
                 if (type == kRem && i == k + 1 && j == k + 1) {  // the next pivot's tile
                     ok = __syncthreads_and(ok);                  // its stores are visible to the whole CTA
-                    if (ok) pivot = int(k) + 1;
+                    if (ok) run_pivot<LB, NQ>(E, int(k) + 1, rowbuf, colbuf);
                 }
             }
-            if (pivot >= 0) run_pivot<LB, NQ>(E, pivot, rowbuf, colbuf);
         }
         __threadfence();
         __syncthreads();
