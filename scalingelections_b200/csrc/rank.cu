@@ -77,13 +77,22 @@ __device__ __forceinline__ void load_pair(const uint32_t* __restrict__ S, int64_
         }
     } else {
         auto at = [&](int r, int c) -> uint32_t { return (r < C && c < C) ? __ldg(S + int64_t(r) * ld + c) : 0u; };
-        constexpr int kStep = WIDE ? 1 : 16;
+        if constexpr (WIDE) {
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const int ra = i0 + ry + 16 * p, ca = j0 + (WIDE ? 4 : 1) * cx;
-            const int rb = j0 + ry + 16 * p, cb = i0 + (WIDE ? 4 : 1) * cx;
-            a[p] = make_uint4(at(ra, ca), at(ra, ca + kStep), at(ra, ca + 2 * kStep), at(ra, ca + 3 * kStep));
-            b[p] = make_uint4(at(rb, cb), at(rb, cb + kStep), at(rb, cb + 2 * kStep), at(rb, cb + 3 * kStep));
+            for (int p = 0; p < 4; ++p) {
+                const int ra = i0 + ry + 16 * p, ca = j0 + 4 * cx;
+                const int rb = j0 + ry + 16 * p, cb = i0 + 4 * cx;
+                a[p] = make_uint4(at(ra, ca), at(ra, ca + 1), at(ra, ca + 2), at(ra, ca + 3));
+                b[p] = make_uint4(at(rb, cb), at(rb, cb + 1), at(rb, cb + 2), at(rb, cb + 3));
+            }
+        } else {
+            const int c0 = col_at<WIDE>(cx, 0), c1 = col_at<WIDE>(cx, 1), c2 = col_at<WIDE>(cx, 2), c3 = col_at<WIDE>(cx, 3);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const int ra = i0 + ry + 16 * p, rb = j0 + ry + 16 * p;
+                a[p] = make_uint4(at(ra, j0 + c0), at(ra, j0 + c1), at(ra, j0 + c2), at(ra, j0 + c3));
+                b[p] = make_uint4(at(rb, i0 + c0), at(rb, i0 + c1), at(rb, i0 + c2), at(rb, i0 + c3));
+            }
         }
     }
 }
