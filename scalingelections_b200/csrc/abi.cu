@@ -52,6 +52,17 @@ void set_error(const char* fmt, ...) {
 void clear_error() { g_last_error[0] = 0; }
 
 se_status_t raise_smem_limit(const void* fn, int bytes, const char* what) {
+    // What this thread has seen done, one entry per slot: a small call asks for a few kernels each time.
+    struct Seen {
+        const void* fn = nullptr;
+        unsigned long long ctx = 0;
+        int bytes = 0;
+    };
+    constexpr unsigned kSlots = 64;
+    thread_local Seen seen[kSlots];
+    const unsigned long long ctx = current_context_id();  // one device's; a new context has no limits raised
+    Seen& slot = seen[(reinterpret_cast<uintptr_t>(fn) >> 4) % kSlots];
+    if (ctx && slot.fn == fn && slot.ctx == ctx && slot.bytes == bytes) return SE_OK;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
@@ -60,17 +71,20 @@ se_status_t raise_smem_limit(const void* fn, int bytes, const char* what) {
     }
     return host_guard([&]() -> se_status_t {  // the cache's insert can throw std::bad_alloc
         static std::mutex m;
-        static std::set<std::tuple<const void*, int, unsigned long long, int>> done;  // a new context has none
+        static std::set<std::tuple<const void*, int, unsigned long long, int>> done;
         std::lock_guard<std::mutex> lock(m);
-        const unsigned long long ctx = current_context_id();
-        if (done.count({fn, dev, ctx, bytes})) return SE_OK;
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            set_error("cannot raise the shared-memory limit of %s: %s", what, cudaGetErrorString(e));
-            return SE_ERR_CUDA;
+        if (!ctx || !done.count({fn, dev, ctx, bytes})) {
+            const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                set_error("cannot raise the shared-memory limit of %s: %s", what, cudaGetErrorString(e));
+                return SE_ERR_CUDA;
+            }
+            done.insert({fn, dev, current_context_id(), bytes});
         }
-        done.insert({fn, dev, current_context_id(), bytes});
+        slot.fn = fn;
+        slot.ctx = ctx;
+        slot.bytes = bytes;
         return SE_OK;
     });
 }

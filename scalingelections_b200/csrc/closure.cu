@@ -1370,7 +1370,8 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
     // That launch may give way where other kernels hold the SMs that it needs. A call that waits
     // then runs the launches; one that only queues has queued gated launches behind it, so it needs
     // room for them, and a second pivot block for that form to apply.
-    if (resident_named && phase_ms == nullptr &&
+    if (resident_named && phase_ms == nullptr && C <= resident::max_candidates(lb) &&
+        work_bytes >= resident::workspace_bytes(C, lb) &&
         (sync || resident::single_cta(C) || (C > kT && work_bytes >= plan(C, lb).flow_total))) {
         if (se_status_t st = prepare_launches(lane_bits)) return st;
         for (;;) {
