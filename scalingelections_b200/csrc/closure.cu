@@ -1367,8 +1367,8 @@ se_status_t closure_run(const uint32_t* d_pref, int64_t ld_pref, int C, uint32_t
     int mode = mode_override >= 0 ? mode_override : g_closure_mode.load();
     bool resident_named = false;
     if (mode == 0) automatic_mode(C, &resident_named);
-    // Matrices that fit the SMs' register files close in one launch (closure_resident.cu): 1.4 to
-    // 2.1 times faster than the launches below at every size that it takes (its shapes' table).
+    // Matrices that fit the SMs' register files close in one launch (closure_resident.cu): 1.26 to 2.1
+    // times as fast as the launches below from 129 candidates on, 1.05 to 1.65 times below (its shapes' table).
     // That launch may give way where other kernels hold the SMs that it needs. A call that waits
     // then runs the launches; one that only queues has queued gated launches behind it, so it needs
     // room for them, and a second pivot block for that form to apply.

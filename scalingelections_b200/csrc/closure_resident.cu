@@ -954,7 +954,13 @@ template <int LB, int CB, int OCC, int ST> Shape shape() {
 //   32-bit lanes   C = 1024             1x2 329   2x1 373             launches 593
 //                  C = 1344                       3x1 610   2x2 820   launches 777
 //                  C = 1500                       4x1 879             launches 866: not taken
-// Two CTAs per SM take no more than 80 registers a thread, and in 32-bit lanes three stages.
+// The shapes taken, with the check-in, against the launches (a whole call): 16-bit lanes C = 16 50 / 67, 64 52 / 66,
+// 65 62 / 67, 128 63 / 66, 129 66 / 105, 256 81 / 134, 512 118 / 228, 768 156 / 324, 1024 220 / 423, 1088 237 /
+// 481, 1344 418 / 602, 1536 489 / 700; 32-bit lanes C = 16 43 / 71, 64 53 / 71, 128 68 / 71, 129 70 / 134, 256
+// 95 / 184, 512 156 / 322, 768 217 / 457, 1024 325 / 589, 1344 612 / 770.
+// Two CTAs per SM take no more than 80 registers a thread, and in 32-bit lanes three stages. All shapes but
+// the first spill a little (stores / loads, bytes: 16-bit 1x2 48 / 104, 2x2 76 / 176; 32-bit 1x1 40 / 96, 1x2
+// 232 / 556, 3x1 112 / 348): the helper warps' registers are allocated at the compute warps' count.
 const Shape* shapes(int lane_bits, int* n) {
     static const Shape s16[] = {shape<16, 1, 1, 4>(), shape<16, 1, 2, 4>(), shape<16, 2, 2, 4>()};
     static const Shape s32[] = {shape<32, 1, 1, 4>(), shape<32, 1, 2, 3>(), shape<32, 3, 1, 4>()};
