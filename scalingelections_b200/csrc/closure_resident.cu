@@ -1085,7 +1085,9 @@ Hold::~Hold() {
     if (!flight) return;
     std::lock_guard<std::mutex> lock(static_cast<Flights*>(flights)->m);
     Flight& x = *static_cast<Flight*>(flight);
-    if (--x.held == 0 && !queued) x.ctas = 0;  // the call has waited for its stream
+    // The call has waited for its stream. (Where another thread queued on that stream meanwhile, its launch is
+    // no longer counted; two launches that then do not fit together settle it by the check-in.)
+    if (--x.held == 0 && !queued) x.ctas = 0;
 }
 
 // The check-in's limit, of the calling thread's launches. Once the CTAs that there is room for spin, the
